@@ -48,6 +48,14 @@ def compute_device(device) -> torch.device:
     return torch.device("cuda", torch.cuda.current_device() if torch.cuda.is_available() else 0)
 
 
+def made_now(device) -> bool:
+    """Whether device state just made on the current stream may be kept for later calls.
+
+    In a stream capture it is only recorded: it exists while that graph runs, so the caller uses it and
+    keeps nothing."""
+    return not torch.cuda.is_current_stream_capturing()
+
+
 class FFTStage:
     """Shapes and launchers for one (grid_shape, image_shape) pair."""
 
@@ -85,7 +93,7 @@ class FFTStage:
         1024^2 the columns' 32 x 32 stages lose: 16 coils, 512^2 147 / 139 against 127 / 146, 8 coils, 1024^2
         98 / 107 against 138 / 123.
         """
-        key = str(device)
+        key = device.index if device.index is not None else torch.cuda.current_device()
         if key not in self._tw:
             tw = None
             if all(g in line_lengths() and g < 1024 for g in self.grid_shape):
@@ -95,6 +103,8 @@ class FFTStage:
                     _lib.call("pgb_fft_twiddle_tables", g, 0, tw[d].data_ptr(), None, st)
                 _lib.call("pgb_fft_twiddle_tables", *self.grid_shape[-2:], tw[-2].data_ptr(), tw[-1].data_ptr(), st)
                 tw = (tw, np.array([t.data_ptr() for t in tw], dtype=np.uint64))
+                if not made_now(device):
+                    return tw
             self._tw[key] = tw
         return self._tw[key]
 

@@ -122,9 +122,10 @@ class GrogToeplitzOp:
             v = torch.empty(B * C * n[0] * g[1] * g[2], dtype=torch.complex64, device=x.device)
             u = v if n[1] == g[1] else torch.empty(B * C * n[0] * n[1] * g[2], dtype=torch.complex64, device=x.device)
             b, c = (B, C) if smaps is not None else (B * C, 1)
+            tw = st._lines(x.device)
             _lib.call("pgb_toep3d", x.data_ptr(), smaps.data_ptr() if smaps is not None else None,
                       self._psf3[s].data_ptr(), u.data_ptr(), v.data_ptr(), out.data_ptr(), b, c, st._n.ctypes.data,
-                      st._g.ctypes.data, st._lines(x.device)[1].ctypes.data, x.data_ptr() if damp else None, float(damp),
+                      st._g.ctypes.data, tw[1].ctypes.data, x.data_ptr() if damp else None, float(damp),
                       _lib.stream_ptr(x.device))
             return out
         if self._lines is not None:

@@ -27,7 +27,7 @@ class MaskedFFTPlan:
 
 import numpy as np
 
-from .._fftops import FFTStage, as_c64, compute_device, with_torch
+from .._fftops import FFTStage, as_c64, compute_device, made_now, with_torch
 from .._solve import SolveMixin
 
 __all__ = ["MaskedFFTPlan", "MaskedFFT"]
@@ -161,25 +161,27 @@ class MaskedFFT(SolveMixin):
     def __call__(self, x, adjoint=False):
         return self.adjoint(x) if adjoint else self.forward(x)
 
+    def _toeplitz(self):
+        op = self._toep_op
+        if op is None:
+            from .._toep import GrogToeplitzOp
+
+            op = GrogToeplitzOp(self, device=self._cdev)
+            if made_now(self._cdev):
+                self._toep_op = op
+        return op
+
     @with_torch
     def normal(self, image):
         if self.toeplitz:
-            if self._toep_op is None:
-                from .._toep import GrogToeplitzOp
-
-                self._toep_op = GrogToeplitzOp(self, device=self._cdev)
-            return self._toep_op(image)
+            return self._toeplitz()(image)
         return self.adjoint(self.forward(image))
 
     def _normal_into(self, x, out, damp: float = 0.0):
         if self.stack_shape:
             raise NotImplementedError("device CG loop covers unstacked operators")
         if self.toeplitz:
-            if self._toep_op is None:
-                from .._toep import GrogToeplitzOp
-
-                self._toep_op = GrogToeplitzOp(self, device=self._cdev)
-            return self._toep_op._apply_into(x, out, damp)
+            return self._toeplitz()._apply_into(x, out, damp)
         y = self.adjoint(self.forward(x))
         out.copy_(y + damp * x if damp else y)
         return out

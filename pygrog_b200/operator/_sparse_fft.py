@@ -22,7 +22,7 @@ import numpy as np
 import torch
 
 from .. import _ext
-from .._fftops import CellLists, FFTStage, as_c64, compute_device, with_torch
+from .._fftops import CellLists, FFTStage, as_c64, compute_device, made_now, with_torch
 from .._solve import SolveMixin
 
 
@@ -46,20 +46,21 @@ class _StackArrays:
         self.R = int(idx_nat.numel())
         self._stage, self._lists = stage, None
 
-    @property
-    def lists(self) -> CellLists:
-        """The replicas by cell, for the adjoint, and ``w_cell``, their weights."""
-        if self._lists is None:
+    def by_cell(self) -> tuple:
+        """The replicas by cell, for the adjoint, and their weights."""
+        made = self._lists
+        if made is None:
             lists = CellLists(self._stage.grid_shape, self.cellpos, self.w)
-            self.w_cell = self.w[lists.rep].contiguous()
-            self._lists = lists
-        return self._lists
+            made = lists, self.w[lists.rep].contiguous()
+            if made_now(self.w.device):
+                self._lists = made
+        return made
 
     def to_grid(self, sparse: torch.Tensor, B: int, C: int) -> torch.Tensor:
         """Weighted samples ``(B, C, R)`` summed on the grid, FFT order ``(B, C, *grid)``."""
         u = torch.empty(B, C, *self._stage.grid_shape, dtype=torch.complex64, device=sparse.device)
-        lists = self.lists
-        return self._stage.cell_sum(sparse, lists, self.w_cell, u, B, C, int(sparse.shape[-1]))
+        lists, w = self.by_cell()
+        return self._stage.cell_sum(sparse, lists, w, u, B, C, int(sparse.shape[-1]))
 
 
 class SparseFFT(SolveMixin):
@@ -136,16 +137,19 @@ class SparseFFT(SolveMixin):
 
     # ------------------------------------------------------------------
     def _stack_arrays_dev(self, s: int) -> _StackArrays:
-        if self._arrays is None:
+        arrays = self._arrays
+        if arrays is None:
             S = int(np.prod(self.stack_shape)) if self.stack_shape else 1
             idx = self.indices.reshape(S, -1).to(self._cdev)
             sw = self.sqrt_weights.reshape(S, -1).to(self._cdev)
             ip = self.inv_perm.reshape(S, -1).to(self._cdev)
-            self._arrays = [
+            arrays = [
                 _StackArrays(self._stage, torch.gather(idx[k], 0, ip[k]), torch.gather(sw[k], 0, ip[k]))
                 for k in range(S)
             ]
-        return self._arrays[s]
+            if made_now(self._cdev):
+                self._arrays = arrays
+        return arrays[s]
 
     def _stack_arrays(self, s_flat_idx: int):
         """``(indices, sqrt_weights, sort_perm, inv_perm)`` of one stack element."""
@@ -256,15 +260,21 @@ class SparseFFT(SolveMixin):
     # ------------------------------------------------------------------
     # normal operator
     # ------------------------------------------------------------------
+    def _toeplitz(self):
+        op = self._toep_op
+        if op is None:
+            from .._toep import GrogToeplitzOp
+
+            op = GrogToeplitzOp(self, device=self._cdev)
+            if made_now(self._cdev):
+                self._toep_op = op
+        return op
+
     @with_torch
     def normal(self, image):
         """``A^H A image`` (Toeplitz PSF when ``self.toeplitz``, else adjoint(forward))."""
         if self.toeplitz:
-            if self._toep_op is None:
-                from .._toep import GrogToeplitzOp
-
-                self._toep_op = GrogToeplitzOp(self, device=self._cdev)
-            return self._toep_op(image)
+            return self._toeplitz()(image)
         return self.adjoint(self.forward(image))
 
     def _normal_into(self, x: torch.Tensor, out: torch.Tensor, damp: float = 0.0) -> torch.Tensor:
@@ -273,11 +283,7 @@ class SparseFFT(SolveMixin):
         if self.stack_shape:
             raise NotImplementedError("device CG loop covers unstacked operators")
         if self.toeplitz:
-            if self._toep_op is None:
-                from .._toep import GrogToeplitzOp
-
-                self._toep_op = GrogToeplitzOp(self, device=self._cdev)
-            return self._toep_op._apply_into(x, out, damp)
+            return self._toeplitz()._apply_into(x, out, damp)
         C = self._n_coils(x.shape[0] if x.ndim > len(self.image_shape) else 1)
         k = self._forward_core(x.reshape(1, *x.shape), 0, C)
         st = self._stage
@@ -290,11 +296,7 @@ class SparseFFT(SolveMixin):
         if self.stack_shape:
             raise NotImplementedError("frame-batched normal operator covers unstacked operators")
         if self.toeplitz:
-            if self._toep_op is None:
-                from .._toep import GrogToeplitzOp
-
-                self._toep_op = GrogToeplitzOp(self, device=self._cdev)
-            return self._toep_op._apply_frames(x, 0, out, damp)
+            return self._toeplitz()._apply_frames(x, 0, out, damp)
         F = int(x.shape[0])
         C = self._n_coils(x.shape[1] if x.ndim > len(self.image_shape) + 1 else 1)
         k = self._forward_core(x, 0, C)

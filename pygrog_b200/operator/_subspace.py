@@ -36,7 +36,7 @@ import numpy as np
 import torch
 
 from .. import _ext, _lib
-from .._fftops import as_c64, with_torch
+from .._fftops import as_c64, made_now, with_torch
 from .._solve import SolveMixin
 from .._toep import line_normal, line_plan
 
@@ -132,19 +132,24 @@ class SubspaceSparseFFT(SolveMixin):
 
     def _weights(self, s: int):
         """(stack arrays, w = pre_w * sqrt_w natural, w * ortho)."""
-        if s not in self._w2:
+        made = self._w2.get(s)
+        if made is None:
             a = self._base._stack_arrays_dev(s)
             w2 = (a.w * a.w).contiguous()
-            self._w2[s] = (a, w2, (w2 * self._base._stage.ortho).contiguous())
-        return self._w2[s]
+            made = (a, w2, (w2 * self._base._stage.ortho).contiguous())
+            if made_now(self._cdev):
+                self._w2[s] = made
+        return made
 
     def _cell_lists(self, s: int):
         """The replicas by cell, with their weights and encoding indices (``csrc/cell_sum.cu``)."""
-        if s not in self._lists:
-            a = self._base._stack_arrays_dev(s)
-            lists = a.lists
-            self._lists[s] = (lists, (a.w_cell * a.w_cell).contiguous(), self._tidx[lists.rep].contiguous())
-        return self._lists[s]
+        made = self._lists.get(s)
+        if made is None:
+            lists, w = self._base._stack_arrays_dev(s).by_cell()
+            made = (lists, (w * w).contiguous(), self._tidx[lists.rep].contiguous())
+            if made_now(self._cdev):
+                self._lists[s] = made
+        return made
 
     def _split(self, x: torch.Tensor, single_ndim: int):
         prefix = tuple(int(v) for v in x.shape[: x.ndim - single_ndim])
@@ -224,9 +229,12 @@ class SubspaceSparseFFT(SolveMixin):
         return self.adjoint(x) if adjoint else self.forward(x)
 
     def _toeplitz(self):
-        if self._toep_op is None:
-            self._toep_op = SubspaceToeplitzOp(self, device=self._cdev)
-        return self._toep_op
+        op = self._toep_op
+        if op is None:
+            op = SubspaceToeplitzOp(self, device=self._cdev)
+            if made_now(self._cdev):
+                self._toep_op = op
+        return op
 
     @with_torch
     def normal(self, coeffs):
