@@ -49,11 +49,15 @@ def compute_device(device) -> torch.device:
 
 
 def made_now(device) -> bool:
-    """Whether device state just made on the current stream may be kept for later calls.
+    """Whether device state just made on the current stream may be kept for later calls, which may come from any
+    stream: it is complete on return.
 
     In a stream capture it is only recorded: it exists while that graph runs, so the caller uses it and
     keeps nothing."""
-    return not torch.cuda.is_current_stream_capturing()
+    if torch.cuda.is_current_stream_capturing():
+        return False
+    torch.cuda.current_stream(device).synchronize()
+    return True
 
 
 class FFTStage:

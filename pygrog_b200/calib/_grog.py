@@ -35,7 +35,7 @@ import torch
 
 from .. import _lib
 from ._grappa import KernelTable
-from .._fftops import CellLists, FFTStage
+from .._fftops import CellLists, FFTStage, made_now
 from ._plan6 import BrickPlan6, _sm_count, lane_chunk
 
 _DEFAULT_DEVICE = "cuda"
@@ -1042,7 +1042,8 @@ class GrogInterpolator:
             tc_ops = self._tc_operands() if mode in ("tc", "tc1") else None
             bp = GrogGridder(tgt, idx, rep_w, kw, plan.grid_shape, self._interp_kernel, self._factors,
                              self._nsteps, mode=mode, tc_ops=tc_ops, brick=getattr(self, "gridder_brick", None))
-            self._brick_plans[s] = bp
+            if made_now(self.device):
+                self._brick_plans[s] = bp
         return bp
 
     # -- forward interpolation ------------------------------------------------
