@@ -50,6 +50,15 @@ def _vdot_re64(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
 _CG_ITERS_PER_GRAPH = 5
 
 
+def _as_rhs(b: torch.Tensor, like: torch.Tensor) -> torch.Tensor:
+    """``b`` as ``like.copy_(b)`` would take it (its errors, broadcasting and conversions), itself where the start
+    kernel can read it as it lies."""
+    if (b.shape == like.shape and b.dtype == like.dtype and b.device == like.device and b.stride() == like.stride()
+            and not b.is_conj() and not b.is_neg()):
+        return b
+    return torch.empty_like(like).copy_(b)
+
+
 class DeviceCG:
     """CG state for one frame on the device (FP64 scalars, optional CUDA graph)."""
 
@@ -82,7 +91,7 @@ class DeviceCG:
     def reset(self, AHb: torch.Tensor, x0=None):
         """Start a new solve in the same buffers (a captured iteration graph stays valid)."""
         if x0 is None:
-            b = AHb.contiguous()
+            b = _as_rhs(AHb, self.r)
             _lib.call("pgb_cg_start_batched", b.data_ptr(), self.x.data_ptr(), self.r.data_ptr(), self.p.data_ptr(),
                       self.n, 1, self.tol, self.scal.data_ptr(), self.scratch.data_ptr(),
                       _lib.stream_ptr(self.p.device))
@@ -183,7 +192,7 @@ class BatchedDeviceCG:
         self.F = F
         self.x, self.r, self.p, self.Ap = (t[:F] for t in (self._x, self._r, self._p, self._Ap))
         self.scal = self._scal[:F]
-        b = AHb.to(torch.complex64).contiguous()
+        b = _as_rhs(AHb, self.r)
         _lib.call("pgb_cg_start_batched", b.data_ptr(), self.x.data_ptr(), self.r.data_ptr(), self.p.data_ptr(), self.n,
                   F, self.tol, self.scal.data_ptr(), self.scratch.data_ptr(), _lib.stream_ptr(b.device))
 
