@@ -195,8 +195,11 @@ static int line_axes(int64_t B, int64_t C, int ndim, const int64_t* image, const
   }
   a.n01 = a.n[0] * a.n[1];
   a.g12 = a.g[1] * a.g[2];
-  PGB_REQUIRE(B < (1 << 24) && C < (1 << 24) && B * C * (a.n01 + a.g12) < (int64_t(1) << 31), PGB_ERR_RANGE,
-              "%s: too many planes", who);
+  // blocks of the widest passes: rows, columns of the middle axis (n[0] planes of a coil image), columns of z
+  const int64_t middle = a.n[0] * ((a.g[2] + 7) / 8), z = ndim == 3 ? (a.g12 + 7) / 8 : 0;
+  const int64_t most = a.n01 > middle ? (a.n01 > z ? a.n01 : z) : (middle > z ? middle : z);
+  PGB_REQUIRE(B < (1 << 28) && C < (1 << 28) && B * C < (int64_t(1) << 31) && B * C * most < (int64_t(1) << 31),
+              PGB_ERR_RANGE, "%s: too many planes", who);
   return PGB_OK;
 }
 

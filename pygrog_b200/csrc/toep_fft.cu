@@ -362,8 +362,9 @@ int pgb_toep2d(const void* x, const void* smaps, const float* psf, void* work, v
   PGB_REQUIRE(B >= 0 && C >= 1 && n0 >= 1 && n1 >= 1 && n0 <= L0 && n1 <= L1, PGB_ERR_INVALID, "toep2d: invalid sizes");
   if (B == 0) return PGB_OK;
   PGB_REQUIRE(x && psf && work && out && tw0 && tw1, PGB_ERR_INVALID, "toep2d: null pointer");
-  PGB_REQUIRE(L0 <= 4096 && L1 <= 4096 && B < (1 << 24) && C < (1 << 24) &&
-                  B * C * (K > 0 ? K : 1) * (n0 + L1) < (int64_t(1) << 31),
+  // blocks of the passes: rows, and columns (4 a block with components)
+  PGB_REQUIRE(L0 <= 4096 && L1 <= 4096 && B < (1 << 28) && C < (1 << 28) && B * C < (int64_t(1) << 31) &&
+                  B * C * (K > 0 ? K : 1) * n0 < (int64_t(1) << 31) && B * C * ((L1 + 3) / 4) < (int64_t(1) << 31),
               PGB_ERR_RANGE, "toep2d: too many planes");
   PGB_REQUIRE(K >= 0 && K <= kSubMax, PGB_ERR_UNSUPPORTED, "toep2d: at most %d components", kSubMax);
   const int64_t BC = B * C;
