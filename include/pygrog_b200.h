@@ -469,18 +469,27 @@ PGB_API int pgb_cell_sum(const void* y, const uint32_t* start, const uint32_t* s
                          int64_t K, int64_t R, int ndim, const int64_t* grid_shape, const void* seg,
                          int64_t n_seg, const void* cells, int64_t n_cells, void* part, void* stream);
 
+/* u[bc, cellpos[r]] += w[r] * data[bc, r] for bc < BC (u pre-zeroed by the
+ * caller); entries with cellpos outside [0,G) or w == 0 are skipped. */
+PGB_API int pgb_sparse_scatter(const void* data, const int32_t* cellpos, const float* w, void* u,
+                               int64_t BC, int64_t R, int64_t G, void* stream);
+
 /* out[bc, r] = w[r] * U[bc, cellpos[r]] (0 for cellpos outside [0,G)). */
 PGB_API int pgb_sparse_gather(const void* U, const int32_t* cellpos, const float* w, void* out,
                               int64_t BC, int64_t R, int64_t G, void* stream);
 
-/* Low-rank subspace transfers (replace the per-(coil, component) gather
- * loops of gadgets/_subspace.py:424-508 and the PSF matvec of
+/* Low-rank subspace transfers (replace the per-(coil, component) scatter /
+ * gather loops of gadgets/_subspace.py:311-508 and the PSF matvec of
  * _toep/_sub_toep.py:236-303).  y (B, C, R) natural sample order, u / U
  * (B, K, C, G) FFT-order grids, basis (K, T) complex64, tidx (R) int32 index
  * along the encoding axis, cellpos (R) int32 FFT-order cell, w (R) float.
+ *   scatter: u[b,k,c,cell_r] += w_r * basis[k,t_r] * y[b,c,r]
  *   gather:  y[b,c,r] = w_r * sum_k conj(basis[k,t_r]) * U[b,k,c,cell_r]
  *   psf_apply_kk (in place): U[b,k,c,g] = sum_k' P[g,k,k'] * U[b,k',c,g],
  *            P (G, K, K) complex64, K <= 16. */
+PGB_API int pgb_subspace_scatter(const void* y, const int32_t* cellpos, const float* w, const int32_t* tidx,
+                                 const void* basis, void* u, int64_t B, int64_t C, int64_t K, int64_t T,
+                                 int64_t R, int64_t G, void* stream);
 PGB_API int pgb_subspace_gather(const void* U, const int32_t* cellpos, const float* w, const int32_t* tidx,
                                 const void* basis, void* out, int64_t B, int64_t C, int64_t K, int64_t T,
                                 int64_t R, int64_t G, void* stream);

@@ -106,6 +106,7 @@ _SIGS = {
     "pgb_cell_sum": [
         _vp, _vp, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _i64, _i64, _i64, _i32, _vp, _vp, _i64, _vp, _i64, _vp, _vp,
     ],
+    "pgb_sparse_scatter": [_vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp],
     "pgb_sparse_gather": [_vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp],
     "pgb_psf_apply": [_vp, _vp, _i64, _i64, _vp],
     "pgb_fft_shift": [_vp, _vp, _vp, _i64, _i32, _vp, _f32, _i32, _vp],
@@ -124,6 +125,7 @@ _SIGS = {
     "pgb_axpy": [_vp, _vp, _f32, _i64, _vp],
     "pgb_grog_grid_v8": [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _i64, _i64, _vp, _vp],
     "pgb_grog_degrid_v8": [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _i64, _i64, _vp, _vp, _vp, _i64, _vp],
+    "pgb_subspace_scatter": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i64, _vp],
     "pgb_subspace_gather": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i64, _vp],
     "pgb_psf_apply_kk": [_vp, _vp, _i64, _i64, _i64, _i64, _vp],
     "pgb_dot_f64_batched": [_vp, _vp, _i64, _i64, _vp, _vp, _i32, _i32, _vp],

@@ -120,6 +120,35 @@ __global__ void fft_combine_kernel(const float2* __restrict__ v, const float2* _
   }
 }
 
+// u[b, c, cellpos[r]] += w[r] * data[b, c, r]  (warp-aggregated atomics; u zeroed by caller)
+// plane bc = b * C + c in y (grid-stride), replicas r in x.  An entry of the C API for grids in any state;
+// the operators sum by cell (cell_sum.cu)
+__global__ void __launch_bounds__(256) sparse_scatter_kernel(const float2* __restrict__ data,
+                                                             const int32_t* __restrict__ cellpos,
+                                                             const float* __restrict__ w,
+                                                             float2* __restrict__ u, int BC, int64_t R,
+                                                             int64_t G) {
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  for (int bc = blockIdx.y; bc < BC; bc += gridDim.y) {
+    const float2* drow = data + static_cast<int64_t>(bc) * R;
+    for (int64_t base = static_cast<int64_t>(blockIdx.x) * blockDim.x; base < R; base += stride) {
+      const int64_t r = base + threadIdx.x;
+      int64_t key = -1;
+      float2 val = make_float2(0.f, 0.f);
+      if (r < R) {
+        const int32_t cp = cellpos[r];
+        const float ww = w[r];
+        if (cp >= 0 && cp < G && ww != 0.f) {
+          key = static_cast<int64_t>(bc) * G + cp;
+          val = cscale(drow[r], ww);
+        }
+      }
+      const unsigned active = __ballot_sync(0xffffffffu, key >= 0);
+      if (key >= 0) warp_aggregated_add(u, key, val, active);
+    }
+  }
+}
+
 // out[b, c, r] = w[r] * U[b, c, cellpos[r]]: replica r from x, kGatherRows
 // planes bc per block row, whose loads of one position and weight are
 // followed by all planes' loads of the cell.
@@ -255,6 +284,20 @@ int pgb_fft_combine(const void* v, const void* smaps, void* out, int64_t B, int6
       static_cast<const float2*>(v), static_cast<const float2*>(smaps), static_cast<float2*>(out),
       static_cast<int>(B), static_cast<int>(C), s, scale, static_cast<const float2*>(add), add_scale);
   PGB_LAUNCH_CHECK("fft_combine");
+  return PGB_OK;
+}
+
+int pgb_sparse_scatter(const void* data, const int32_t* cellpos, const float* w, void* u, int64_t BC,
+                       int64_t R, int64_t G, void* stream) {
+  clear_error();
+  PGB_REQUIRE(BC >= 0 && R >= 0 && G >= 0, PGB_ERR_INVALID, "sparse_scatter: negative size");
+  if (BC == 0 || R == 0 || G == 0) return PGB_OK;
+  PGB_REQUIRE(data && cellpos && w && u, PGB_ERR_INVALID, "sparse_scatter: null pointer");
+  const unsigned ys = static_cast<unsigned>(BC < 65535 ? BC : 65535);
+  const int xs = grid_for(R, 256, (148 * 16 + ys - 1) / ys);
+  sparse_scatter_kernel<<<dim3(xs, ys), 256, 0, as_stream(stream)>>>(
+      static_cast<const float2*>(data), cellpos, w, static_cast<float2*>(u), static_cast<int>(BC), R, G);
+  PGB_LAUNCH_CHECK("sparse_scatter");
   return PGB_OK;
 }
 

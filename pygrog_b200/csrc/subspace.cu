@@ -1,22 +1,61 @@
-// subspace.cu -- grid to sparse transfer and PSF of the low-rank subspace
-// operator (samples to grid: cell_sum.cu).
+// subspace.cu -- sparse <-> grid transfers of the low-rank subspace operator.
 //
-// Reference: gadgets/_subspace.py (SubspaceSparseFFT._forward_single 424-508)
-// and _toep/_sub_toep.py (SubspaceToeplitzOp, PSF 120-208, apply 236-303).  The reference loops over coils and subspace
+// Reference: gadgets/_subspace.py (SubspaceSparseFFT._adjoint_single 311-400,
+// _forward_single 424-508) and _toep/_sub_toep.py (SubspaceToeplitzOp,
+// PSF 120-208, apply 236-303).  The reference loops over coils and subspace
 // components with one scatter / FFT per (c, k); here one pass reads every
 // sample once for all K components:
 //
+//   scatter: u[b, k, c, cell_r] += w_r * B[k, t_r] * y[b, c, r]
 //   gather:  y[b, c, r] = w_r * sum_k conj(B[k, t_r]) * U[b, k, c, cell_r]
 //   psf:     V[b, k, c, g] = sum_k' P[g, k, k'] * U[b, k', c, g]   (in place)
 //
 // cell_r is the FFT-order grid position, t_r the sample's index along the
 // encoding (time / contrast) axis; samples with cell or t out of range
-// contribute nothing (gather writes 0).
+// contribute nothing (gather writes 0).  The operators sum their samples by
+// cell (cell_sum.cu); the scatter, which adds to a grid in any state and needs
+// no lists, is an entry of the C API.
 #include "common.cuh"
 
 namespace pgb {
 
 constexpr int kMaxK = 32;
+
+__global__ void __launch_bounds__(256) subspace_scatter_kernel(
+    const float2* __restrict__ y, const int32_t* __restrict__ cellpos, const float* __restrict__ w,
+    const int32_t* __restrict__ tidx, const float2* __restrict__ basis, float2* __restrict__ u, int B, int C,
+    int K, int T, int64_t R, int64_t G) {
+  const int64_t total = static_cast<int64_t>(B) * C * R;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  for (int64_t base = static_cast<int64_t>(blockIdx.x) * blockDim.x; base < total; base += stride) {
+    const int64_t t = base + threadIdx.x;
+    bool ok = false;
+    int64_t b = 0, c = 0, cp = 0;
+    int ti = 0;
+    float2 val = make_float2(0.f, 0.f);
+    if (t < total) {
+      const int64_t r = t % R;
+      const int64_t bc = t / R;
+      b = bc / C;
+      c = bc - b * C;
+      cp = cellpos[r];
+      ti = tidx[r];
+      const float ww = w[r];
+      ok = cp >= 0 && cp < G && ti >= 0 && ti < T && ww != 0.f;
+      if (ok) val = cscale(y[t], ww);
+    }
+    for (int k = 0; k < K; ++k) {  // warp-uniform
+      int64_t key = -1;
+      float2 v = make_float2(0.f, 0.f);
+      if (ok) {
+        key = ((b * K + k) * C + c) * G + cp;
+        v = cmul(__ldg(basis + static_cast<int64_t>(k) * T + ti), val);
+      }
+      const unsigned active = __ballot_sync(0xffffffffu, key >= 0);
+      if (key >= 0) warp_aggregated_add(u, key, v, active);
+    }
+  }
+}
 
 __global__ void subspace_gather_kernel(const float2* __restrict__ U, const int32_t* __restrict__ cellpos,
                                        const float* __restrict__ w, const int32_t* __restrict__ tidx,
@@ -70,6 +109,22 @@ __global__ void psf_apply_kk_kernel(float2* __restrict__ U, const float2* __rest
 using namespace pgb;
 
 extern "C" {
+
+int pgb_subspace_scatter(const void* y, const int32_t* cellpos, const float* w, const int32_t* tidx,
+                         const void* basis, void* u, int64_t B, int64_t C, int64_t K, int64_t T, int64_t R,
+                         int64_t G, void* stream) {
+  clear_error();
+  PGB_REQUIRE(B >= 0 && C >= 0 && R >= 0 && G >= 0 && T >= 1 && K >= 1 && K <= kMaxK, PGB_ERR_INVALID,
+              "subspace_scatter: invalid sizes (K must be 1..%d)", kMaxK);
+  if (B == 0 || C == 0 || R == 0 || G == 0) return PGB_OK;
+  PGB_REQUIRE(B * C < (int64_t(1) << 31), PGB_ERR_RANGE, "subspace_scatter: too many frames");
+  PGB_REQUIRE(y && cellpos && w && tidx && basis && u, PGB_ERR_INVALID, "subspace_scatter: null pointer");
+  subspace_scatter_kernel<<<grid_for(B * C * R, 256, 148 * 16), 256, 0, as_stream(stream)>>>(
+      static_cast<const float2*>(y), cellpos, w, tidx, static_cast<const float2*>(basis), static_cast<float2*>(u),
+      static_cast<int>(B), static_cast<int>(C), static_cast<int>(K), static_cast<int>(T), R, G);
+  PGB_LAUNCH_CHECK("subspace_scatter");
+  return PGB_OK;
+}
 
 int pgb_subspace_gather(const void* U, const int32_t* cellpos, const float* w, const int32_t* tidx,
                         const void* basis, void* out, int64_t B, int64_t C, int64_t K, int64_t T, int64_t R,
