@@ -411,7 +411,7 @@ PGB_API int pgb_sample_sum(const void* y, const int32_t* ptr, const float* w, vo
  * index (outside [0, K): zeros).  pgb_grog_expand_order makes both from
  * idx (N * kw) and adds the number of runs of one operator to *runs.  src (N),
  * if not NULL: where sample n lies in data (B, C, stride) (outside: zeros).  The
- * table is 32-byte aligned. */
+ * table is aligned to 32 bytes where C is a multiple of 4, 16 where it is even. */
 PGB_API int pgb_grog_expand_chunk(int64_t N, int64_t C, int64_t kw);
 PGB_API int pgb_grog_expand_order(const int64_t* idx, int64_t N, int kw, int64_t K, int64_t C, uint32_t* order,
                                   int32_t* ent, int32_t* runs, void* stream);

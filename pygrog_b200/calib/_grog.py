@@ -668,6 +668,8 @@ class GrogGridder:
         self.w_cell = self.w[self.lists.rep].contiguous()
         self.ptr = torch.searchsorted(self.samp, torch.arange(N + 1, dtype=torch.int32, device=dev), out_int32=True)
         self.table = torch.as_tensor(table).to(dev).contiguous()
+        if self.table.data_ptr() % 32:  # a view
+            self.table = self.table.clone()
         self.table_h = self.table.conj().transpose(-1, -2).resolve_conj().contiguous()
         self._stage = FFTStage(grid_shape, grid_shape)
         # split_bricks: the cells whose replicas are summed in several parts
@@ -1121,6 +1123,8 @@ class GrogInterpolator:
     def _expand_order(self, s: int, idx: torch.Tensor, C: int, kw: int):
         """Replicas of stack element ``s`` ordered by operator inside each chunk of samples, ``(order, entry)`` of
         ``csrc/grog_expand.cu``, where that pays: ``None`` where a chunk's replicas hardly share operators."""
+        if C % 4 == 0 and self._table_d.data_ptr() % 32:
+            return None  # a view: its rows are not whole 32-byte sectors
         key, orders = (s, C), self.__dict__.setdefault("_orders", {})
         if key not in orders:
             if torch.cuda.is_current_stream_capturing():

@@ -244,7 +244,9 @@ int pgb_grog_expand_sorted(const void* data, int64_t N, const int32_t* src, int6
   if (N == 0 || B == 0) return PGB_OK;
   PGB_REQUIRE(data && order && ent && table && out, PGB_ERR_INVALID, "grog_expand_sorted: null pointer");
   PGB_REQUIRE(B <= 65535, PGB_ERR_RANGE, "grog_expand_sorted: batch must be <= 65535");
-  PGB_REQUIRE(reinterpret_cast<uintptr_t>(table) % 32 == 0, PGB_ERR_INVALID, "grog_expand_sorted: table not 32-byte aligned");
+  const int align = C % 4 == 0 ? 32 : C % 2 == 0 ? 16 : 8;  // of the operator loads
+  PGB_REQUIRE(reinterpret_cast<uintptr_t>(table) % align == 0, PGB_ERR_INVALID,
+              "grog_expand_sorted: table not %d-byte aligned", align);
   int ns, cg;
   ns = pgb_grog_expand_chunk(N, C, kw);
   if (ns > 0) expand_shape(N, C, kw, ns, cg);
