@@ -645,9 +645,8 @@ class GrogGridder:
         self.plan = BrickPlan(target_idx, interp_idx, rep_weight, kw, grid_shape, **kwargs)
         self.adj_plan = self.plan
 
-    @staticmethod
-    def _can_order(target_idx, kw, grid_shape, K) -> bool:
-        return int(np.prod(grid_shape)) < 2**31 and target_idx.numel() < 2**31 and K < 2**31 - 1
+    def _can_order(self, target_idx, kw, grid_shape, K) -> bool:
+        return (self.C <= 32 and int(np.prod(grid_shape)) < 2**31 and target_idx.numel() < 2**31 and K < 2**31 - 1)
 
     def _init_ordered(self, target_idx, interp_idx, rep_weight, kw, grid_shape, table):
         """The plan's valid replicas, ascending by sample: their operators' order (``csrc/grog_expand.cu``), the
@@ -656,7 +655,7 @@ class GrogGridder:
         tgt = target_idx.reshape(-1)
         N = tgt.numel() // kw
         if not self._can_order(tgt, kw, grid_shape, int(table.shape[0])):
-            raise ValueError("ordered kernels need grids, replica counts and tables below 2^31")
+            raise ValueError("ordered kernels need C <= 32 and grids, replica counts and tables below 2^31")
         r = torch.nonzero(tgt >= 0).squeeze(1)
         V, C, K = int(r.numel()), self.C, int(table.shape[0])
         order = expand_order(interp_idx.reshape(-1)[r], K, C, 1, always=True)
