@@ -242,10 +242,10 @@ def check_tc_timeouts(what: str) -> None:
 
 
 def stream_ptr(device=None) -> int:
-    index = getattr(device, "index", None)
-    if index is None:  # no device, its name, or "cuda" without a number
-        return torch.cuda.current_stream(device).cuda_stream
-    return torch._C._cuda_getCurrentRawStream(index)
+    """The current stream of ``device`` (anything torch takes as one)."""
+    if isinstance(device, torch.device) and device.index is not None and device.type == "cuda":
+        return torch._C._cuda_getCurrentRawStream(device.index)
+    return torch.cuda.current_stream(device).cuda_stream
 
 
 def ptr(t: torch.Tensor | None) -> int | None:
