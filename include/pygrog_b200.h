@@ -453,6 +453,7 @@ PGB_API int pgb_fft_combine(const void* v, const void* smaps, void* out, int64_t
  *   basis == NULL: u[b,c,cell] = sum w y[b,c,src],          u (B, C, grid)
  *   else:          u[b,k,c,cell] = sum w basis[k,tix] y[b,c,src],
  *                  u (B, K, C, grid), basis (K, T) complex64, K <= 32.
+ * Replicas with src outside y or tix outside the basis add nothing.
  * Every cell of the grid is written.  Long lists are summed by segment:
  * pgb_cell_segments fills seg and cells, int32 rows of 4 with at most
  * pgb_cell_bounds(listed replicas) of each (rows past the counts are zero or

@@ -66,6 +66,12 @@ __global__ void __launch_bounds__(kCellThreads)
         ww[q] = w[at];
         if constexpr (SUB) t[q] = tix[at];
       }
+      if constexpr (SUB) {  // no such encoding: the replica adds nothing
+        if (static_cast<unsigned>(t[q]) >= static_cast<unsigned>(T)) {
+          r = 0xffffffffu;
+          t[q] = 0;
+        }
+      }
       if (r >= R) ww[q] = 0.f;  // past the end, or fewer samples than the plan has
 #pragma unroll
       for (int j = 0; j < CB; ++j) v[q][j] = r < R && j < nc ? yb[j * R + r] : make_float2(0.f, 0.f);
@@ -265,8 +271,8 @@ int pgb_cell_sum(const void* y, const uint32_t* start, const uint32_t* src, cons
   CellGrid g;
   const int st = cell_grid(ndim, grid_shape, g);
   if (st) return st;
-  PGB_REQUIRE(B >= 0 && C >= 0 && K >= 1 && K <= 32 && R >= 0 && T >= 0 && (basis != nullptr || K == 1), PGB_ERR_INVALID,
-              "cell_sum: invalid sizes (K must be 1..32)");
+  PGB_REQUIRE(B >= 0 && C >= 0 && K >= 1 && K <= 32 && R >= 0 && T >= 0 && (basis != nullptr ? T >= 1 : K == 1), PGB_ERR_INVALID,
+              "cell_sum: invalid sizes (K must be 1..32, T at least 1)");
   if (B == 0 || C == 0) return PGB_OK;
   PGB_REQUIRE(u && start && (y || R == 0) && (!basis || tix), PGB_ERR_INVALID, "cell_sum: null pointer");
   const int64_t G = static_cast<int64_t>(g.g[0]) * g.g[1] * g.g[2];
