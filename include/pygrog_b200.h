@@ -419,6 +419,15 @@ PGB_API int pgb_grog_expand_sorted(const void* data, int64_t N, const int32_t* s
                                    const uint32_t* order, const int32_t* ent, const void* table, int64_t K,
                                    int64_t C, int64_t B, void* out, void* stream);
 
+/* The shifts of the ordered gridder: out[b,:,v] = T[e_v] data[b,:,src[v]] for V
+ * replicas (order and ent as above with kw = 1, src as above, M positions).
+ * second == NULL: T is table (K, C, C).  Else, up to 16 coils, T[e] = second[e % n]
+ * table[e / n], the factors applied in turn; with adjoint the two are given
+ * transposed and T[e] = table[e / n] second[e % n]. */
+PGB_API int pgb_grog_shift(const void* data, int64_t M, const int32_t* src, int64_t V, const uint32_t* order,
+                           const int32_t* ent, const void* table, int64_t K, const void* second, int64_t n,
+                           int adjoint, int64_t C, int64_t B, void* out, void* stream);
+
 /* =====================================================================
  * SparseFFT / MaskedFFT / Toeplitz stages around cuFFT
  * (operator/_sparse_fft.py:574-621, 741-789, 1154-1177;

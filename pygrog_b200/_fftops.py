@@ -77,14 +77,15 @@ class FFTStage:
         self._g = np.ascontiguousarray(self.grid_shape, dtype=np.int64)
         self._n = np.ascontiguousarray(self.image_shape, dtype=np.int64)
         self.ortho = 1.0 / math.sqrt(self.G)
-        self._tw = {}
+        self.__setstate__({})
 
     def __getstate__(self):
-        # the twiddles go with their addresses: a copy makes its own
+        # the twiddles and the shape go with their addresses: a copy makes its own
         return {**self.__dict__, "_tw": {}}
 
     def __setstate__(self, state):
         self.__dict__.update(state, _tw={})
+        self._g_ptr = self._g.ctypes.data
 
     # -- transforms with the coil maps ----------------------------------------
     def _lines(self, device):
@@ -207,13 +208,13 @@ class FFTStage:
     def cell_sum(self, data, lists, w, u, B, C, R, tix=None, basis=None):
         """Grid ``u (B, [K,] C, *grid)`` in FFT order from samples ``data (B, C, R)``; every cell is written.
         ``w`` (and ``tix``): the weights (and basis columns) of the listed replicas."""
-        K, T = (int(v) for v in basis.shape) if basis is not None else (1, 0)
-        n_seg, n_cells = int(lists.seg.shape[0]), int(lists.cells.shape[0])
-        part = torch.empty(B * K * C * n_seg if n_cells else 0, dtype=torch.complex64, device=u.device)
+        K, T = basis.shape if basis is not None else (1, 0)
+        n_seg, n_cells = lists.seg.shape[0], lists.cells.shape[0]
+        part = torch.empty(B * K * C * n_seg, dtype=torch.complex64, device=u.device) if n_cells else None
         _lib.call("pgb_cell_sum", data.data_ptr(), lists.start.data_ptr(), lists.src.data_ptr(), w.data_ptr(),
                   tix.data_ptr() if tix is not None else None, basis.data_ptr() if basis is not None else None, T,
-                  u.data_ptr(), B, C, K, R, self.ndim, self._g.ctypes.data, lists.seg.data_ptr(), n_seg,
-                  lists.cells.data_ptr(), n_cells, part.data_ptr(), _lib.stream_ptr(u.device))
+                  u.data_ptr(), B, C, K, R, self.ndim, self._g_ptr, lists.seg.data_ptr(), n_seg,
+                  lists.cells.data_ptr(), n_cells, part.data_ptr() if n_cells else None, _lib.stream_ptr(u.device))
         return u
 
     @staticmethod

@@ -97,6 +97,7 @@ _SIGS = {
     "pgb_grog_expand_chunk": [_i64, _i64, _i64],
     "pgb_grog_expand_order": [_vp, _i64, _i32, _i64, _i64, _vp, _vp, _vp, _vp],
     "pgb_grog_expand_sorted": [_vp, _i64, _vp, _i64, _i32, _vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp],
+    "pgb_grog_shift": [_vp, _i64, _vp, _i64, _vp, _vp, _vp, _i64, _vp, _i64, _i32, _i64, _i64, _vp, _vp],
     "pgb_sample_sum": [_vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp],
     "pgb_fft_expand": [_vp, _vp, _vp, _i64, _i64, _i32, _vp, _vp, _f32, _i32, _vp],
     "pgb_fft_combine": [_vp, _vp, _vp, _i64, _i64, _i32, _vp, _vp, _f32, _vp, _f32, _vp],

@@ -521,9 +521,6 @@ class GrogGridder:
         if brick is not None:
             cand = (tuple(brick),)
         self.tc = None
-        if mode == "ordered":
-            self._init_ordered(target_idx, interp_idx, rep_weight, kw, grid_shape, table)
-            return
         if mode in ("tc", "tc1"):
             self._init_tc(mode, tc_ops, target_idx, interp_idx, rep_weight, kw, grid_shape, cand, lib)
             return
@@ -540,7 +537,7 @@ class GrogGridder:
         chosen = None
         self.sub_cap = None
         self.fwd6 = None  # (brick, sub_cap, factored) of the v6 forward used with the v8 adjoint
-        if mode in (None, "v8", "v8pair") and C <= 16:
+        if mode in (None, "ordered", "v8", "v8pair") and C <= 16:
             n_out_f = int(factors[0].shape[0]) if factors is not None else None
             for sub in (256, 192, 128):
                 for br in cand:
@@ -564,7 +561,7 @@ class GrogGridder:
                             break
                     if self.fwd6 is not None:
                         break
-        if chosen is None and mode in (None, "v6") and C <= 16:
+        if chosen is None and mode in (None, "ordered", "v6") and C <= 16:
             n_out_f = int(factors[0].shape[0]) if factors is not None else None
             for sub in (128, 96, 64):
                 for br in cand:
@@ -584,10 +581,11 @@ class GrogGridder:
         # 192 k x 8 56 / 32 against 43 / 36, 600 k x 13 381 / 275 against 308 / 274, 2.6 M x 12 (249 MB) 676 / 449
         # against 1005 / 1161; "global": 102 k x 32 837 / 831 against 127 / 113, 1.5 M x 16 1413 / 1135 against
         # 1062 / 1171.
-        if mode is None and brick is None and self._can_order(target_idx, kw, grid_shape, K):
-            if chosen is None or int((target_idx >= 0).sum()) * C * 8 <= 64 * 2**20:
-                self._init_ordered(target_idx, interp_idx, rep_weight, kw, grid_shape, table)
-                return
+        pays = mode is None and brick is None and self._can_order(target_idx, kw, grid_shape, K)
+        if mode == "ordered" or pays and (chosen is None or int((target_idx >= 0).sum()) * C * 8 <= 64 * 2**20):
+            self._init_ordered(target_idx, interp_idx, rep_weight, kw, grid_shape, table,
+                               factors if chosen is not None and chosen[2] else None)
+            return
         if chosen is None:
             if mode in ("v6", "v8", "v8pair"):
                 raise ValueError(f"{mode} kernels need C <= 16 and a table that fits shared memory")
@@ -648,7 +646,7 @@ class GrogGridder:
     def _can_order(self, target_idx, kw, grid_shape, K) -> bool:
         return (self.C <= 32 and int(np.prod(grid_shape)) < 2**31 and target_idx.numel() < 2**31 and K < 2**31 - 1)
 
-    def _init_ordered(self, target_idx, interp_idx, rep_weight, kw, grid_shape, table):
+    def _init_ordered(self, target_idx, interp_idx, rep_weight, kw, grid_shape, table, factors):
         """The plan's valid replicas, ascending by sample: their operators' order (``csrc/grog_expand.cu``), the
         lists by cell (``csrc/cell_sum.cu``) and the ranges by sample."""
         dev = target_idx.device
@@ -658,30 +656,41 @@ class GrogGridder:
             raise ValueError("ordered kernels need C <= 32 and grids, replica counts and tables below 2^31")
         r = torch.nonzero(tgt >= 0).squeeze(1)
         V, C, K = int(r.numel()), self.C, int(table.shape[0])
-        order = expand_order(interp_idx.reshape(-1)[r], K, C, 1, always=True)
+        order, entry = expand_order(interp_idx.reshape(-1)[r], K, C, 1, always=True)
         self.mode, self.brick, self.sub_cap, self.fwd6, self.plan2 = "ordered", None, None, None, None
-        self.order, self.entry = order
+        self.order, self.entry = order, entry
         self.samp, self.cell = (r // kw).to(torch.int32), tgt[r].to(torch.int32)
         self.w = rep_weight.reshape(-1)[r].to(torch.float32).contiguous()
         self.lists = CellLists(grid_shape, self.cell, self.w)
         self.w_cell = self.w[self.lists.rep].contiguous()
         self.ptr = torch.searchsorted(self.samp, torch.arange(N + 1, dtype=torch.int32, device=dev), out_int32=True)
-        self.table = torch.as_tensor(table).to(dev).contiguous()
-        if self.table.data_ptr() % 32:  # a view
-            self.table = self.table.clone()
-        self.table_h = self.table.conj().transpose(-1, -2).resolve_conj().contiguous()
+        # operators, or the factors where the brick kernels apply those (a whole table of ill-conditioned factors is less
+        # exact: 297^2 radial scan, 6 coils, 10,201 operators, error of the grid 2.3e-7 against 0.96e-7), and the
+        # adjoint's
+        outer, inner = (None, table) if factors is None else factors
+        self.K, self.n_outer = K, 1 if outer is None else int(outer.shape[0])
+        self.ops = [None if t is None else torch.as_tensor(t).to(dev).contiguous() for t in (inner, outer)]
+        self.ops = [t.clone() if t is not None and t.data_ptr() % 32 else t for t in self.ops]  # views
+        self.ops_h = [None if t is None else t.conj().transpose(-1, -2).resolve_conj().contiguous() for t in self.ops]
         self._stage = FFTStage(grid_shape, grid_shape)
         # split_bricks: the cells whose replicas are summed in several parts
         self.plan = self.adj_plan = SimpleNamespace(n_valid=V, split_bricks=self.lists.cells[:, 0])
 
-    def _shift(self, x: torch.Tensor, src: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
-        """Each valid replica's operator of ``table`` on ``x (B, C, M)`` at ``src``, ``(B, C, n_valid)``."""
+    def _ordered(self, x: torch.Tensor, out: torch.Tensor, adjoint: bool) -> None:
+        """Every valid replica's operator (adjoint: transposed) on its sample (cell), summed by cell (sample)."""
         B, C, M = x.shape
-        V = int(src.numel())
+        V = self.plan.n_valid
+        st = _lib.stream_ptr(x.device)
         y = torch.empty(B, C, V, dtype=x.dtype, device=x.device)
-        _lib.call("pgb_grog_expand_sorted", x.data_ptr(), V, src.data_ptr(), M, 1, self.order.data_ptr(),
-                  self.entry.data_ptr(), table.data_ptr(), table.shape[0], C, B, y.data_ptr(), _lib.stream_ptr(x.device))
-        return y
+        inner, outer = self.ops_h if adjoint else self.ops
+        _lib.call("pgb_grog_shift", x.data_ptr(), M, (self.cell if adjoint else self.samp).data_ptr(), V,
+                  self.order.data_ptr(), self.entry.data_ptr(), inner.data_ptr(), self.K,
+                  None if outer is None else outer.data_ptr(), self.n_outer, adjoint, C, B, y.data_ptr(), st)
+        if adjoint:
+            _lib.call("pgb_sample_sum", y.data_ptr(), self.ptr.data_ptr(), self.w.data_ptr(), out.data_ptr(),
+                      out.shape[-1], V, B * C, st)
+        else:
+            self._stage.cell_sum(y, self.lists, self.w_cell, out, B, C, V)
 
     def _init_tc(self, mode, tc_ops, target_idx, interp_idx, rep_weight, kw, grid_shape, cand, lib):
         """Tensor-core gridder (``csrc/grog_tc.cu``): sample-ordered v6 plans
@@ -773,11 +782,10 @@ class GrogGridder:
     def forward(self, data: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
         """``out (B, C, G)`` <- fused gridding of ``data (B, C, N)``."""
         B, C, N = data.shape
-        G = out.shape[-1]
         if self.mode == "ordered":
-            y = self._shift(data, self.samp, self.table)
-            self._stage.cell_sum(y, self.lists, self.w_cell, out, B, C, int(y.shape[-1]))
+            self._ordered(data, out, False)
             return out
+        G = out.shape[-1]
         bp = self.plan
         st = _lib.stream_ptr(data.device)
         if self.tc is not None:
@@ -803,13 +811,11 @@ class GrogGridder:
     def adjoint(self, grid: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
         """``out (B, C, N)`` <- adjoint of :meth:`forward` applied to ``grid (B, C, G)``."""
         B, C, G = grid.shape
+        if self.mode == "ordered":
+            self._ordered(grid, out, True)
+            return out
         N = out.shape[-1]
         st = _lib.stream_ptr(grid.device)
-        if self.mode == "ordered":
-            y = self._shift(grid, self.cell, self.table_h)
-            _lib.call("pgb_sample_sum", y.data_ptr(), self.ptr.data_ptr(), self.w.data_ptr(), out.data_ptr(), N,
-                      int(y.shape[-1]), B * C, st)
-            return out
         bp = self.adj_plan
         zs = bp.zero_src.data_ptr() if bp.zero_src.numel() else None
         if self.tc is not None:

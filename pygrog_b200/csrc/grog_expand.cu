@@ -21,8 +21,8 @@
 //
 // The bound is then the FP32 multiply-add rate (4 C^2 a replica) and the
 // operator loads, one wavefront per distinct operator of a warp and 16 bytes.
-// The sum over the input coils runs in the same order as in sample order: the
-// same bits.
+// The expansion's sum over the input coils runs in the same order as in sample
+// order: the same bits.
 #include "common.cuh"
 
 namespace pgb {
@@ -39,12 +39,57 @@ __device__ __forceinline__ void load_sector(const float2* p, float2 (&t)[4]) {
       : "l"(p));
 }
 
-template <int C>
+// One row of an operator times x, in PART partial sums over the input coils.  One:
+// the bits of the sample order.  Two: the brick kernels' sums, for the factors.
+// Four, for the adjoint of a whole table: shorter chains of FP32 roundings, which
+// keep degrid's error at the brick kernels' (2-D, up to 10 coils, ratio of the
+// errors against FP64 0.97 on average with four, 1.07 with one).
+template <int C, int PART>
+__device__ __forceinline__ float2 row_dot(const float2* __restrict__ T, const float2 (&x)[C]) {
+  float2 y[PART] = {};
+  if constexpr (C % 4 == 0) {
+#pragma unroll
+    for (int q = 0; q < C / 4; ++q) {
+      float2 t[4];
+      load_sector(T + 4 * q, t);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) cfma(y[j % PART], t[j], x[4 * q + j]);
+    }
+  } else if constexpr (C % 2 == 0) {
+#pragma unroll
+    for (int q = 0; q < C / 2; ++q) {
+      const float4 t = __ldg(reinterpret_cast<const float4*>(T) + q);
+      cfma(y[2 * q % PART], make_float2(t.x, t.y), x[2 * q]);
+      cfma(y[(2 * q + 1) % PART], make_float2(t.z, t.w), x[2 * q + 1]);
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < C; ++c) cfma(y[c % PART], __ldg(T + c), x[c]);
+  }
+  if constexpr (PART == 4) return cadd(cadd(y[0], y[1]), cadd(y[2], y[3]));
+  else if constexpr (PART == 2) return cadd(y[0], y[1]);
+  else return y[0];
+}
+
+// The operators of a table, or (FACT) of two factors, table[e / n] applied first
+// and second[e % n] to its result, or the other way round (swap): in turn, where
+// the brick kernels do so, since the whole table of smooth coils' factors rounds
+// away what they keep (errors up to 3.6 times theirs).  Twice the products, but
+// on few operators: 33 k replicas of 8 coils (10,201 operators of 2 x 101
+// factors) 26 / 22 us for grid / degrid against 24 / 19 with the whole table,
+// 1.2 M of 11 coils in 3-D 416 / 449 against 572 / 643, of 12 coils 498 / 550
+// against 444 / 541.
+struct ShiftTable {
+  const float2* table;
+  const float2* second;
+  int K, n, swap;
+};
+
+template <int C, int PART, bool FACT>
 __global__ void __launch_bounds__(kExpThreads, 2)
     grog_expand_sorted_kernel(const float2* __restrict__ data, int64_t N, const int32_t* __restrict__ src,
                               int64_t stride, int kw, const uint32_t* __restrict__ order,
-                              const int32_t* __restrict__ ent, const float2* __restrict__ table, int64_t K,
-                              float2* __restrict__ out, int NS, int CG) {
+                              const int32_t* __restrict__ ent, ShiftTable tb, float2* __restrict__ out, int NS, int CG) {
   extern __shared__ float2 smem[];
   float2* xs = smem;           // (C, NS) samples
   float2* stage = smem + C * NS;  // (CG, NS * kw) results in sample order
@@ -62,6 +107,18 @@ __global__ void __launch_bounds__(kExpThreads, 2)
       xs[c * NS + i] = at >= 0 && at < stride ? dat[c * stride + at] : make_float2(0.f, 0.f);
     }
   __syncthreads();
+  if constexpr (FACT) {  // one replica a sample: its first product takes the sample's place
+    for (int i = threadIdx.x; i < nrep; i += kExpThreads) {
+      const int l = order[base + i] & 0xffffu, e = ent[base + i];
+      float2 x[C];
+#pragma unroll
+      for (int c = 0; c < C; ++c) x[c] = xs[c * NS + l];
+      const int at = e >= 0 && e < tb.K ? (tb.swap ? e % tb.n : e / tb.n) : 0;
+      const float2* T = (tb.swap ? tb.second : tb.table) + static_cast<int64_t>(at) * C * C;
+#pragma unroll 4
+      for (int c = 0; c < C; ++c, T += C) xs[c * NS + l] = row_dot<C, PART>(T, x);
+    }
+  }
   for (int g0 = 0; g0 < C; g0 += CG) {
     const int ng = min(CG, C - g0);
     for (int i = threadIdx.x; i < nrep; i += kExpThreads) {
@@ -70,32 +127,12 @@ __global__ void __launch_bounds__(kExpThreads, 2)
       float2 x[C];
 #pragma unroll
       for (int c = 0; c < C; ++c) x[c] = xs[c * NS + n];
-      const bool ok = e >= 0 && e < K;
-      const float2* T = table + (static_cast<int64_t>(ok ? e : 0) * C + g0) * C;
+      const bool ok = e >= 0 && e < tb.K;
+      int at = ok ? e : 0;
+      if constexpr (FACT) at = tb.swap ? at / tb.n : at % tb.n;
+      const float2* T = (FACT && !tb.swap ? tb.second : tb.table) + (static_cast<int64_t>(at) * C + g0) * C;
 #pragma unroll 4  // the operator rows of four coils in flight
-      for (int co = 0; co < ng; ++co, T += C) {
-        float2 y = make_float2(0.f, 0.f);
-        if constexpr (C % 4 == 0) {
-#pragma unroll
-          for (int q = 0; q < C / 4; ++q) {
-            float2 t[4];
-            load_sector(T + 4 * q, t);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) cfma(y, t[j], x[4 * q + j]);
-          }
-        } else if constexpr (C % 2 == 0) {
-#pragma unroll
-          for (int q = 0; q < C / 2; ++q) {
-            const float4 t = __ldg(reinterpret_cast<const float4*>(T) + q);
-            cfma(y, make_float2(t.x, t.y), x[2 * q]);
-            cfma(y, make_float2(t.z, t.w), x[2 * q + 1]);
-          }
-        } else {
-#pragma unroll
-          for (int c = 0; c < C; ++c) cfma(y, __ldg(T + c), x[c]);
-        }
-        stage[co * SR + l] = ok ? y : make_float2(0.f, 0.f);
-      }
+      for (int co = 0; co < ng; ++co, T += C) stage[co * SR + l] = ok ? row_dot<C, PART>(T, x) : make_float2(0.f, 0.f);
     }
     __syncthreads();
     for (int co = 0; co < ng; ++co)
@@ -232,45 +269,79 @@ int pgb_sample_sum(const void* y, const int32_t* ptr, const float* w, void* out,
   return PGB_OK;
 }
 
-int pgb_grog_expand_sorted(const void* data, int64_t N, const int32_t* src, int64_t stride, int kw,
-                           const uint32_t* order, const int32_t* ent, const void* table, int64_t K, int64_t C, int64_t B,
-                           void* out, void* stream) {
+static int expand_sorted(const void* data, int64_t N, const int32_t* src, int64_t stride, int kw, const uint32_t* order,
+                         const int32_t* ent, const void* table, int64_t K, const void* second, int64_t n,
+                         int adjoint, int64_t C, int64_t B, void* out, void* stream, const char* who) {
   clear_error();
   if (!src) stride = N;
-  PGB_REQUIRE(stride >= 0, PGB_ERR_INVALID, "grog_expand_sorted: invalid sizes");
-  PGB_REQUIRE(C >= 1 && C <= 32, PGB_ERR_UNSUPPORTED, "grog_expand_sorted: ncoils must be 1..32, got %lld",
-              (long long)C);
-  PGB_REQUIRE(N >= 0 && B >= 0 && kw >= 1 && K >= 1, PGB_ERR_INVALID, "grog_expand_sorted: invalid sizes");
+  PGB_REQUIRE(stride >= 0, PGB_ERR_INVALID, "%s: invalid sizes", who);
+  const int cmax = second ? 16 : 32;
+  PGB_REQUIRE(C >= 1 && C <= cmax, PGB_ERR_UNSUPPORTED, "%s: ncoils must be 1..%d, got %lld", who, cmax, (long long)C);
+  PGB_REQUIRE(N >= 0 && B >= 0 && kw >= 1 && K >= 1 && (!second || (n >= 1 && K % n == 0 && K < (int64_t(1) << 31))),
+              PGB_ERR_INVALID, "%s: invalid sizes", who);
   if (N == 0 || B == 0) return PGB_OK;
-  PGB_REQUIRE(data && order && ent && table && out, PGB_ERR_INVALID, "grog_expand_sorted: null pointer");
-  PGB_REQUIRE(B <= 65535, PGB_ERR_RANGE, "grog_expand_sorted: batch must be <= 65535");
+  PGB_REQUIRE(data && order && ent && table && out, PGB_ERR_INVALID, "%s: null pointer", who);
+  PGB_REQUIRE(B <= 65535, PGB_ERR_RANGE, "%s: batch must be <= 65535", who);
   const int align = C % 4 == 0 ? 32 : C % 2 == 0 ? 16 : 8;  // of the operator loads
-  PGB_REQUIRE(reinterpret_cast<uintptr_t>(table) % align == 0, PGB_ERR_INVALID,
-              "grog_expand_sorted: table not %d-byte aligned", align);
+  PGB_REQUIRE(reinterpret_cast<uintptr_t>(table) % align == 0 && reinterpret_cast<uintptr_t>(second) % align == 0,
+              PGB_ERR_INVALID, "%s: table not %d-byte aligned", who, align);
   int ns, cg;
   ns = pgb_grog_expand_chunk(N, C, kw);
   if (ns > 0) expand_shape(N, C, kw, ns, cg);
-  PGB_REQUIRE(ns > 0, PGB_ERR_UNSUPPORTED, "grog_expand_sorted: kw=%d too large for the staging tile", kw);
+  PGB_REQUIRE(ns > 0, PGB_ERR_UNSUPPORTED, "%s: kw=%d too large for the staging tile", who, kw);
   const size_t smem = sizeof(float2) * ns * (C + static_cast<int64_t>(cg) * kw);
   const int64_t blocks = (N + ns - 1) / ns;
-  PGB_REQUIRE(blocks < (int64_t(1) << 31), PGB_ERR_RANGE, "grog_expand_sorted: too many samples");
+  PGB_REQUIRE(blocks < (int64_t(1) << 31), PGB_ERR_RANGE, "%s: too many samples", who);
   const dim3 grd(static_cast<unsigned>(blocks), static_cast<unsigned>(B));
+  const ShiftTable tb{static_cast<const float2*>(table), static_cast<const float2*>(second),
+                      static_cast<int>(K < INT32_MAX ? K : INT32_MAX), static_cast<int>(n), adjoint};
   cudaStream_t s = as_stream(stream);
-  switch (C) {
-#define X(CC)                                                                                                    \
-  case CC: {                                                                                                     \
-    allow_smem<grog_expand_sorted_kernel<CC>>(227 * 1024);                                                       \
-    grog_expand_sorted_kernel<CC><<<grd, kExpThreads, smem, s>>>(static_cast<const float2*>(data), N, src, stride, kw, order, ent,           \
-                                     static_cast<const float2*>(table), K, static_cast<float2*>(out), ns, cg);   \
-  } break;
-    X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) X(17) X(18) X(19) X(20)
-    X(21) X(22) X(23) X(24) X(25) X(26) X(27) X(28) X(29) X(30) X(31) X(32)
-#undef X
-    default:
-      break;
+  const auto go = [&](auto launch) {
+    launch(static_cast<const float2*>(data), N, src, stride, kw, order, ent, tb, static_cast<float2*>(out), ns, cg);
+  };
+#define Y(CC, P, F)                                                              \
+  {                                                                              \
+    allow_smem<grog_expand_sorted_kernel<CC, P, F>>(227 * 1024);                 \
+    go([&](auto... a) { grog_expand_sorted_kernel<CC, P, F><<<grd, kExpThreads, smem, s>>>(a...); }); \
   }
-  PGB_LAUNCH_CHECK("grog_expand_sorted");
+  if (second) {
+    switch (C) {
+#define X(CC) \
+  case CC:    \
+    Y(CC, 2, true) break;
+      X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
+#undef X
+    }
+  } else {
+    switch (C) {
+#define X(CC)                            \
+  case CC:                               \
+    if (adjoint) Y(CC, 4, false)         \
+    else Y(CC, 1, false) break;
+      X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) X(17) X(18) X(19) X(20)
+      X(21) X(22) X(23) X(24) X(25) X(26) X(27) X(28) X(29) X(30) X(31) X(32)
+#undef X
+    }
+  }
+#undef Y
+  PGB_LAUNCH_CHECK(who);
   return PGB_OK;
+}
+
+int pgb_grog_expand_sorted(const void* data, int64_t N, const int32_t* src, int64_t stride, int kw,
+                           const uint32_t* order, const int32_t* ent, const void* table, int64_t K, int64_t C, int64_t B,
+                           void* out, void* stream) {
+  return expand_sorted(data, N, src, stride, kw, order, ent, table, K, nullptr, 0, 0, C, B, out, stream,
+                       "grog_expand_sorted");
+}
+
+int pgb_grog_shift(const void* data, int64_t M, const int32_t* src, int64_t V, const uint32_t* order, const int32_t* ent,
+                   const void* table, int64_t K, const void* second, int64_t n, int adjoint, int64_t C, int64_t B,
+                   void* out, void* stream) {
+  clear_error();
+  PGB_REQUIRE(src || V == 0, PGB_ERR_INVALID, "grog_shift: null pointer");
+  return expand_sorted(data, V, src, M, 1, order, ent, table, K, second, n, adjoint, C, B, out, stream,
+                       "grog_shift");
 }
 
 }  // extern "C"
