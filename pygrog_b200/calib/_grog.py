@@ -26,6 +26,7 @@ from __future__ import annotations
 
 __all__ = ["GrogInterpolator", "GrogPlan", "BrickPlan", "GrogGridder"]
 
+import functools
 import math
 import os
 from types import SimpleNamespace
@@ -473,14 +474,19 @@ def _pack_axis_indices(bp: BrickPlan6, nsteps: int, ndim: int) -> None:
     bp.meta[:, 1] = y.to(torch.int32)
 
 
+_ORDERED_BYTES = 64 * 2**20  # shifted replicas of the ordered kernels at a time: they stay in L2
+
+
 class GrogGridder:
     """Fused GROG gridding operator for one trajectory: brick plans + tables.
 
     Kernel families (chosen from the shared-memory budget of one CTA):
       ``"ordered"``   C <= 32: the shifted replicas in the order of their
                       operators, then summed by cell (adjoint: gathered,
-                      shifted, summed by sample); the FP32 default while the
-                      replicas stay in L2, and above 16 coils;
+                      shifted, summed by sample); the FP32 default of small
+                      plans and where no table fits shared memory (a call
+                      with more frames than that pays for takes the family
+                      it stands in for, ``_order_limit``);
       ``"tc"``        C <= 32: eigen-factored table as a chain of dense
                       coil matrices on the tensor cores (bf16x3 split
                       products, FP32 accumulate) with per-replica phases;
@@ -489,7 +495,7 @@ class GrogGridder:
                       streams, replicas ordered (outer, inner, cell) so
                       operator loads are conflict-free or broadcast; the
                       forward sums each cell's replicas without atomics
-                      (the FP32 default of large 3-D plans);
+                      (the FP32 default of large plans and batches);
       ``"v8pair"``    the v8 adjoint with the v6 forward;
       ``"v6"``        C <= 16: operator-stationary slots (outer factor rows
                       in registers along sorted runs, inner factor or whole
@@ -574,18 +580,14 @@ class GrogGridder:
                         break
                 if chosen is not None:
                     break
-        # The ordered kernels write and read the shifted replicas once more than the brick kernels but fill the GPU
-        # on any trajectory: faster while those replicas stay in L2, and always than the table through L1/L2.
-        # Measured (valid replicas x coils; grid / degrid, us, brick against ordered): radial 33 k x 8 46 / 31
-        # against 15 / 12, 179 k x 16 90 / 76 against 81 / 77, spiral 197 k x 16 100 / 138 against 88 / 69, 3-D
-        # 192 k x 8 56 / 32 against 43 / 36, 600 k x 13 381 / 275 against 308 / 274, 2.6 M x 12 (249 MB) 676 / 449
-        # against 1005 / 1161; "global": 102 k x 32 837 / 831 against 127 / 113, 1.5 M x 16 1413 / 1135 against
-        # 1062 / 1171.
-        pays = mode is None and brick is None and self._can_order(target_idx, kw, grid_shape, K)
-        if mode == "ordered" or pays and (chosen is None or int((target_idx >= 0).sum()) * C * 8 <= 64 * 2**20):
-            self._init_ordered(target_idx, interp_idx, rep_weight, kw, grid_shape, table,
-                               factors if chosen is not None and chosen[2] else None)
-            return
+        if mode == "ordered" or mode is None and brick is None and self._can_order(target_idx, kw, grid_shape, K):
+            other = chosen or ("global", None, False)
+            if self._init_ordered(target_idx, interp_idx, rep_weight, kw, grid_shape, table,
+                                  factors if other[2] else None, None if mode == "ordered" else other[:2]):
+                if mode is None:
+                    self._make_other = functools.partial(GrogGridder, target_idx, interp_idx, rep_weight, kw, grid_shape,
+                                                         table, factors, nsteps, mode=other[0], chunk=chunk)
+                return
         if chosen is None:
             if mode in ("v6", "v8", "v8pair"):
                 raise ValueError(f"{mode} kernels need C <= 16 and a table that fits shared memory")
@@ -646,9 +648,34 @@ class GrogGridder:
     def _can_order(self, target_idx, kw, grid_shape, K) -> bool:
         return (self.C <= 32 and int(np.prod(grid_shape)) < 2**31 and target_idx.numel() < 2**31 and K < 2**31 - 1)
 
-    def _init_ordered(self, target_idx, interp_idx, rep_weight, kw, grid_shape, table, factors):
+    def _order_limit(self, other: tuple, run: float) -> float:
+        """Replicas (frames times the plan's) up to which the ordered kernels are the faster ones, against the family
+        and brick ``other`` that the plan would have without them; ``run``: replicas that share an operator in a chunk.
+
+        They write and read the shifted replicas once more than the others but fill the GPU on any trajectory, so
+        they win where the others are short of work, and lose at length to the brick kernels, which read no
+        operator from L2 (a run of 4 halves that traffic).  Measured (1,347 plans and batches, coils 4 to 32; time
+        of grid and degrid, other / ordered): brick kernels, 3-D, 12 coils: 29 k 2.33, 80 k 1.52, 144 k 1.17, 250 k
+        0.86, 1.2 M 0.62; 2-D, 8 coils, 10,201 operators: 33 k 2.00, 2 frames 1.39, 4 frames 1.15, 16 frames 0.85,
+        179 k 0.95; spirals of 8 coils, runs of 12 and 8: 197 k 1.44, 246 k 1.21; 2-D, 16 coils, run 2.9: 90 k
+        1.40, 179 k 0.95.  Where no more than the smallest 3-D brick fits beside the tables (13 coils), in which most
+        of the work is on its faces, the brick kernels lose throughout: 144 k 1.59, 2.7 M 1.09, 16 frames of it 1.01.
+        The table through L1/L2 loses to short runs of whole sectors (C a multiple of 8) and to long runs
+        throughout (16 / 24 / 32 coils in 3-D at 1.2 M 1.50 / 1.62 / 1.57; 2-D above 1.15).  Else it wins at
+        length, the sooner the more lanes its groups of C fill: 15 coils 420 k 1.47, 800 k 0.82; 31 coils 420 k
+        1.06, 1.2 M 0.71; 20 coils 420 k 1.50, 2 frames 1.19, 1.2 M 0.97.
+        """
+        family, brick = other
+        if family != "global":
+            return math.inf if brick == self.BRICKS3[-1] else 256e3 if run >= 4 else 150e3
+        if self.C % 8 == 0 or run >= 2.5:
+            return math.inf
+        return 500e3 if 32 // self.C * self.C >= 28 else 1e6
+
+    def _init_ordered(self, target_idx, interp_idx, rep_weight, kw, grid_shape, table, factors, other) -> bool:
         """The plan's valid replicas, ascending by sample: their operators' order (``csrc/grog_expand.cu``), the
-        lists by cell (``csrc/cell_sum.cu``) and the ranges by sample."""
+        lists by cell (``csrc/cell_sum.cu``) and the ranges by sample.  False, with nothing made, where the
+        family ``other`` is the faster one already for one frame; ``max_batch``: the frames up to which it is not."""
         dev = target_idx.device
         tgt = target_idx.reshape(-1)
         N = tgt.numel() // kw
@@ -656,9 +683,18 @@ class GrogGridder:
             raise ValueError("ordered kernels need C <= 32 and grids, replica counts and tables below 2^31")
         r = torch.nonzero(tgt >= 0).squeeze(1)
         V, C, K = int(r.numel()), self.C, int(table.shape[0])
-        order, entry = expand_order(interp_idx.reshape(-1)[r], K, C, 1, always=True)
+        limit = math.inf if other is None else self._order_limit(other, math.inf)
+        if V > limit:
+            return False
+        order, entry, runs = expand_order(interp_idx.reshape(-1)[r], K, C, 1, always=True)
+        if other is not None:
+            limit = self._order_limit(other, V / max(1, int(runs)))
+        if V > limit:
+            return False
+        self.max_batch = math.inf if V == 0 else limit / V
         self.mode, self.brick, self.sub_cap, self.fwd6, self.plan2 = "ordered", None, None, None, None
         self.order, self.entry = order, entry
+        self._other = self._make_other = None
         self.samp, self.cell = (r // kw).to(torch.int32), tgt[r].to(torch.int32)
         self.w = rep_weight.reshape(-1)[r].to(torch.float32).contiguous()
         self.lists = CellLists(grid_shape, self.cell, self.w)
@@ -675,11 +711,29 @@ class GrogGridder:
         self._stage = FFTStage(grid_shape, grid_shape)
         # split_bricks: the cells whose replicas are summed in several parts
         self.plan = self.adj_plan = SimpleNamespace(n_valid=V, split_bricks=self.lists.cells[:, 0])
+        return True
+
+    def _other_gridder(self) -> "GrogGridder | None":
+        """The family that an ordered default stands in for, for batches above ``max_batch``: made at the first of
+        them; none in a capture before."""
+        other = self._other
+        if other is None and not torch.cuda.is_current_stream_capturing():
+            other = self._make_other()
+            if made_now(self.w.device):
+                self._other = other
+        return other
 
     def _ordered(self, x: torch.Tensor, out: torch.Tensor, adjoint: bool) -> None:
-        """Every valid replica's operator (adjoint: transposed) on its sample (cell), summed by cell (sample)."""
+        """Every valid replica's operator (adjoint: transposed) on its sample (cell), summed by cell (sample).
+
+        A batch is taken in frames whose shifted replicas stay in L2 together: the workspace stays small too."""
         B, C, M = x.shape
         V = self.plan.n_valid
+        n = max(1, _ORDERED_BYTES // (8 * C * V + 1))
+        if B > n:
+            for b in range(0, B, n):
+                self._ordered(x[b : b + n], out[b : b + n], adjoint)
+            return
         st = _lib.stream_ptr(x.device)
         y = torch.empty(B, C, V, dtype=x.dtype, device=x.device)
         inner, outer = self.ops_h if adjoint else self.ops
@@ -783,6 +837,8 @@ class GrogGridder:
         """``out (B, C, G)`` <- fused gridding of ``data (B, C, N)``."""
         B, C, N = data.shape
         if self.mode == "ordered":
+            if B > self.max_batch and (other := self._other_gridder()) is not None:
+                return other.forward(data, out)
             self._ordered(data, out, False)
             return out
         G = out.shape[-1]
@@ -812,6 +868,8 @@ class GrogGridder:
         """``out (B, C, N)`` <- adjoint of :meth:`forward` applied to ``grid (B, C, G)``."""
         B, C, G = grid.shape
         if self.mode == "ordered":
+            if B > self.max_batch and (other := self._other_gridder()) is not None:
+                return other.adjoint(grid, out)
             self._ordered(grid, out, True)
             return out
         N = out.shape[-1]
@@ -844,7 +902,7 @@ class GrogGridder:
 
 def expand_order(idx: torch.Tensor, K: int, C: int, kw: int, always: bool = False):
     """``(order, entry)`` int32 arrays of ``pgb_grog_expand_sorted`` for table indices ``idx (N * kw)``, or ``None``
-    where they do not pay (unless ``always``).
+    where they do not pay; with ``always`` these and the count of runs of one operator (on the device).
 
     A lane per replica costs a load per distinct operator of its warp, a slot of ``C`` lanes per replica the
     whole operator: with runs of one operator of at least 3 replicas on average the former wins.  Measured
@@ -862,7 +920,9 @@ def expand_order(idx: torch.Tensor, K: int, C: int, kw: int, always: bool = Fals
     runs = torch.zeros(1, dtype=torch.int32, device=idx.device)
     _lib.call("pgb_grog_expand_order", idx.data_ptr(), R // kw, kw, K, C, order.data_ptr(), entry.data_ptr(),
               runs.data_ptr(), _lib.stream_ptr(idx.device))
-    return (order, entry) if always or R >= 3 * int(runs) else None
+    if always:
+        return order, entry, runs
+    return (order, entry) if R >= 3 * int(runs) else None
 
 
 # ---------------------------------------------------------------------------
