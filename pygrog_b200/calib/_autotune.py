@@ -7,7 +7,9 @@ choice depends on the trajectory's density, the coil count and the table
 size, so it is measured: every candidate (family x brick that fits shared
 memory) is built on the caller's trajectory and timed forward + adjoint with
 CUDA events on random data of the caller's batch size; the fastest is kept on
-the interpolator and cached per problem signature.
+the interpolator and cached per problem signature.  Where an untuned
+interpolator would take the ordered kernels, which have no brick, they are timed
+beside the candidates and left in place if they are the fastest.
 
 Precision gates the families twice.  The tensor-core bf16x3 family
 (``"tc"``) is a candidate only when the caller accepts a relative error of
@@ -68,15 +70,24 @@ def _time(bp, data: torch.Tensor, G: int, reps: int, warmup: int):
     return float(np.median(ts)), kg, out
 
 
+def _install(g, best: dict) -> None:
+    g.gridder_mode, g.gridder_brick = (best["mode"], best["brick"]) if best["installed"] else (None, None)
+
+
 def autotune_gridder(g, batch: int = 1, tolerance: float = 1e-4, families=None, reps: int = 3, warmup: int = 1,
                      use_cache: bool = True) -> dict:
     """Pick the fastest fused gridder for ``g`` (a ``GrogInterpolator`` after
     ``calc_interp_table``) and install it (``g.gridder_mode``, ``g.gridder_brick``).
 
     Returns ``{"mode", "brick", "ms", "trials": [(mode, brick, ms, err), ...],
-    "rejected": [(mode, brick, err), ...], "cached"}``.  ``ms`` is the forward +
-    adjoint time on stack entry 0; ``err`` the larger relative L2 difference of
-    the forward and adjoint outputs from the FP32 reference candidate.
+    "rejected": [(mode, brick, err), ...], "default_ms", "installed", "cached"}``.
+    ``ms`` is the forward + adjoint time on stack entry 0; ``err`` the larger
+    relative L2 difference of the forward and adjoint outputs from the FP32
+    reference candidate.  ``mode`` and ``brick`` are the fastest of the trials;
+    ``default_ms`` is the time of the ordered kernels where they are what the
+    untuned interpolator takes (``None``: they are not, or ``families`` were
+    asked for).  If that is the shortest, ``installed`` is ``None`` and the
+    interpolator stays untuned; else ``installed`` is ``mode``.
     """
     from ._grog import GrogGridder
 
@@ -85,11 +96,12 @@ def autotune_gridder(g, batch: int = 1, tolerance: float = 1e-4, families=None, 
     key = _signature(g, batch, tolerance)
     if use_cache and key in _CACHE:
         best = _CACHE[key]
-        g.gridder_mode, g.gridder_brick = best["mode"], best["brick"]
+        _install(g, best)
         g._brick_plans = None
         return dict(best, cached=True)
     C = int(g._interp_kernel.shape[-1])
     ndim = len(g.plan.grid_shape)
+    untuned = families is None
     if families is None:
         families = ["v8", "v6"] if C <= 16 else ["global"]  # FP32 shared-memory families cover C <= 16
         if C <= 32 and tolerance >= 1e-4:
@@ -148,7 +160,14 @@ def autotune_gridder(g, batch: int = 1, tolerance: float = 1e-4, families=None, 
         raise RuntimeError("autotune_gridder: no candidate gridder fits this problem")
     best["trials"] = trials
     best["rejected"] = rejected
-    g.gridder_mode, g.gridder_brick = best["mode"], best["brick"]
+    best["default_ms"], best["installed"] = None, best["mode"]
+    if untuned:
+        bp = GrogGridder(tgt, idx, rep_w, kw, plan.grid_shape, g._interp_kernel, g._factors, g._nsteps)
+        if bp.mode == "ordered" and batch <= bp.max_batch:
+            best["default_ms"] = _time(bp, data, G, reps, warmup)[0]
+            if best["default_ms"] <= best["ms"]:
+                best["installed"], best_bp = None, bp
+    _install(g, best)
     g._brick_plans = {0: best_bp} if s_total == 1 else None
     if use_cache:
         _CACHE[key] = best
