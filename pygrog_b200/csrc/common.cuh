@@ -38,16 +38,34 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 
 constexpr int kNumSMs = 148;  // B200
 
-// Lets kernel K take `bytes` of dynamic shared memory: set once a device, as
-// the call costs the host about a microsecond of a launch's five.
+// Number of the calling thread's current driver context, never given twice in a
+// process (0: none yet, or the driver does not tell).
+inline unsigned long long context_id() {
+  using CtxGetId = int (*)(void*, unsigned long long*);
+  static const CtxGetId get = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &fn, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      return reinterpret_cast<CtxGetId>(fn);
+    cudaGetLastError();
+    return static_cast<CtxGetId>(nullptr);
+  }();
+  unsigned long long id = 0;
+  return get != nullptr && get(nullptr, &id) == 0 ? id : 0;
+}
+
+// Lets kernel K take `bytes` of dynamic shared memory.  The call costs the host
+// about a microsecond of a launch's five, so it is left out while the context is
+// the one that K was last allowed it in (the limit belongs to a context: another
+// device's, another one of this device, the one after cudaDeviceReset).
 template <auto K>
 inline void allow_smem(int bytes) {
-  static std::atomic<uint64_t> done{0};
-  int dev = 64;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64 || !(done.load(std::memory_order_relaxed) >> dev & 1)) {
-    const cudaError_t e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess && dev < 64) done.fetch_or(uint64_t(1) << dev, std::memory_order_relaxed);
-  }
+  static std::atomic<unsigned long long> allowed{0};
+  const unsigned long long ctx = context_id();
+  if (ctx != 0 && allowed.load(std::memory_order_relaxed) == ctx) return;
+  if (cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
+    allowed.store(ctx, std::memory_order_relaxed);
 }
 
 // Launch that need not wait for the stream's previous kernel to be flushed
