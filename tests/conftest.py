@@ -18,6 +18,15 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (B200) and libpygrog_b200.so")
 
 
+def pytest_collection_modifyitems(items):
+    """The test that needs the reference's compiled CPU kernels (``oracle/_ref``, built from its sources) runs last
+    where they have not been built: a run that stops at the first failure has then run the others."""
+    from oracle.build_ref import built_path
+
+    if built_path() is None:
+        items.sort(key=lambda it: it.name.startswith("test_config0_matches_reference_cpu_path"))
+
+
 def golden(name: str) -> dict:
     with np.load(GOLDEN / name, allow_pickle=False) as z:
         return {k: z[k] for k in z.files}
