@@ -307,6 +307,24 @@ struct Line {
   }
 };
 
+// Lines per block of the row kernel: about 256 threads and at most 40 KB.
+template <class F>
+constexpr int rows_per_block() {
+  constexpr int by_threads = F::T >= 192 ? 1 : 256 / F::T, by_smem = 5120 / F::SZ;  // 40 KB
+  return by_smem < 1 ? 1 : by_threads < by_smem ? by_threads : by_smem;
+}
+
+// Groups of threads an output row's coils are dealt to (a block of 256
+// threads, of 160 where a line takes two stages and its threads hold more).
+// Measured at (length, coils): groups for 512 threads against these,
+// 640, 16: 20.4 -> 16.4 us; 768, 24: 54 -> 26; 384, 24: 21.4 -> 15.9;
+// 256, 16: 7.7 -> 6.4: smaller blocks leave the tail of the last wave short.
+template <class F>
+constexpr int coil_groups() {
+  constexpr int n = F::R3 > 1 ? 256 : 160;
+  return 2 * F::T > n ? 1 : n / F::T;
+}
+
 // Groups of T threads, at most `most`, to which an output row's C coils are
 // dealt.  With few rows: as many as keep them busy, unless the last turn
 // would leave over a tenth of their time unused (16 coils on 3 or 2 groups of

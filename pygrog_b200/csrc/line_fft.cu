@@ -20,19 +20,13 @@
 namespace pgb {
 namespace fft {
 
-template <class F>
-constexpr int line_rows_per_block() {
-  constexpr int by_threads = F::T >= 192 ? 1 : 256 / F::T, by_smem = 5120 / F::SZ;  // 40 KB
-  return by_smem < 1 ? 1 : by_threads < by_smem ? by_threads : by_smem;
-}
-
 // U[b, c, q, :] = FFT of row q of S_c x_b, natural order: the slots pass
 // through shared memory once more, so that rows are written whole.
 template <class F>
-__global__ void __launch_bounds__(F::T* line_rows_per_block<F>())
+__global__ void __launch_bounds__(F::T* rows_per_block<F>())
     line_rows_kernel(const float2* __restrict__ x, const float2* __restrict__ smaps, float2* __restrict__ U, int C,
                      int n0, Centre ce, int64_t units, const float2* __restrict__ tw) {
-  __shared__ float2 smr[line_rows_per_block<F>()][F::SZ];
+  __shared__ float2 smr[rows_per_block<F>()][F::SZ];
   float2* sm = smr[threadIdx.y];
   grid_wait();
   const int t = threadIdx.x;
@@ -66,16 +60,10 @@ __global__ void __launch_bounds__(F::T* line_rows_per_block<F>())
   }
 }
 
-template <class F>
-constexpr int line_groups() {  // as coil_groups of toep_fft.cu
-  constexpr int n = F::R3 > 1 ? 256 : 160;
-  return 2 * F::T > n ? 1 : n / F::T;
-}
-
 // One image row of one frame per block, its coils dealt to groups of threads
 // and summed in group order (toep_out_kernel), from rows in natural order.
 template <class F>
-__global__ void __launch_bounds__(F::T* line_groups<F>())
+__global__ void __launch_bounds__(F::T* coil_groups<F>())
     line_out_kernel(const float2* __restrict__ U, const float2* __restrict__ smaps, float2* __restrict__ out, int C,
                     int n0, Centre ce, float scale, const float2* __restrict__ add, float add_scale,
                     const float2* __restrict__ tw) {
@@ -151,7 +139,7 @@ __global__ void __launch_bounds__(F::T* line_groups<F>())
 template <class F>
 int launch_line_rows(const float2* x, const float2* S, float2* U, int64_t B, int C, int n0, int n1, const float2* tw,
                      cudaStream_t s) {
-  constexpr int FB = line_rows_per_block<F>();
+  constexpr int FB = rows_per_block<F>();
   const int64_t units = B * n0 * C;
   const Centre ce{n1, F::L / 2 - (F::L - n1) / 2};
   launch_chained(line_rows_kernel<F>, static_cast<unsigned>((units + FB - 1) / FB), dim3(F::T, FB), 0, s, x, S, U, C, n0,
@@ -163,7 +151,7 @@ int launch_line_rows(const float2* x, const float2* S, float2* U, int64_t B, int
 template <class F>
 int launch_line_out(const float2* U, const float2* S, float2* out, int64_t B, int C, int n0, int n1, float scale,
                     const float2* add, float add_scale, const float2* tw, cudaStream_t s) {
-  constexpr int GM = line_groups<F>();
+  constexpr int GM = coil_groups<F>();
   const int G = coil_group_count(C, F::T, GM, B * n0);
   const size_t smem = sizeof(float2) * F::SZ * G;
   auto k = line_out_kernel<F>;

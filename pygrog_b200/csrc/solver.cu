@@ -291,8 +291,9 @@ __global__ void cg_update_p_kernel(float2* __restrict__ p, const float2* __restr
 // and 4.5 + 5.4 + 3.6 us at 320^2 for 0.1 and 0.8 MB a vector, and two gaps
 // between launches.  Here a cluster of CL blocks takes a frame: the two sums
 // go through the blocks' shared memories in rank order (so results do not
-// vary) with two cluster barriers, and p, Ap and r (E elements a thread; r from
-// the first pass on where that leaves no spills) stay in registers.
+// vary) with two cluster barriers, and p, Ap and r (E elements a thread) stay in
+// registers; r is read in the first pass for E <= 8 (128 registers, 8 and 20
+// bytes spilled) and in the second for E = 20 (128, 72 bytes).
 constexpr int kStepThreads = 512;
 
 template <int CL, int E>

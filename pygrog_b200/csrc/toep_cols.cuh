@@ -7,7 +7,13 @@
 namespace pgb {
 namespace fft {
 
-constexpr int kSubMax = 5;  // components of the subspace form
+// Components of the subspace form: a block has F::T x 4 threads for each. 5 of
+// them (640 threads at most) leave 96 registers a thread and next to no spills
+// (12 to 24 bytes at L = 800, 960 and 1024). Built for 8 (64 registers, 0.4 to
+// 2.5 KB spilled at L = 384 and more) the smaller ranks pay: 8 coils, L = 384,
+// image 192 x 192, an application of 4 components 51 -> 96 us, of 5 72 -> 126
+// (cuFFT: 182, 183).
+constexpr int kSubMax = 5;
 
 // The column transforms, the PSF and their inverse in place on the planes U
 // (BC, n0, L1); PGB_ERR_UNSUPPORTED if the length L0 is not built.

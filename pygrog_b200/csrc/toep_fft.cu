@@ -30,13 +30,6 @@
 namespace pgb {
 namespace fft {
 
-// Lines per block of the row kernel: about 256 threads and at most 40 KB.
-template <class F>
-constexpr int rows_per_block() {
-  constexpr int by_threads = F::T >= 192 ? 1 : 256 / F::T, by_smem = 5120 / F::SZ;  // 40 KB
-  return by_smem < 1 ? 1 : by_threads < by_smem ? by_threads : by_smem;
-}
-
 template <class F, bool HALF>
 __global__ void __launch_bounds__(F::T* rows_per_block<F>())
     toep_rows_kernel(const float2* __restrict__ x, const float2* __restrict__ smaps, float2* __restrict__ U, int C,
@@ -70,17 +63,6 @@ __global__ void __launch_bounds__(F::T* rows_per_block<F>())
     float2* ur = U + ((b * C + c) * n0 + q) * F::L + t;
     unroll<0, F::RL>([&](auto j) { ur[j * F::NL] = o[j]; });
   }
-}
-
-// Groups of threads an output row's coils are dealt to (a block of 256
-// threads, of 160 where a line takes two stages and its threads hold more).
-// Measured at (length, coils): groups for 512 threads against these,
-// 640, 16: 20.4 -> 16.4 us; 768, 24: 54 -> 26; 384, 24: 21.4 -> 15.9;
-// 256, 16: 7.7 -> 6.4: smaller blocks leave the tail of the last wave short.
-template <class F>
-constexpr int coil_groups() {
-  constexpr int n = F::R3 > 1 ? 256 : 160;
-  return 2 * F::T > n ? 1 : n / F::T;
 }
 
 // One image row of one frame per block; its coils are dealt to blockDim.y

@@ -346,7 +346,7 @@ class SubspaceMaskedFFT(SubspaceSparseFFT):
         return (o.reshape(Bt, self.K, C, st.G) * self._phi_conj).sum(1)
 
 
-_LINE_K = 5  # components the line-FFT kernels hold together (csrc/toep_fft.cu)
+_LINE_K = 5  # components the line-FFT kernels hold together (kSubMax of csrc/toep_cols.cuh, with the reason)
 
 
 def _pack_hermitian(P: torch.Tensor) -> torch.Tensor:
