@@ -40,7 +40,12 @@ struct CellGrid {
 // 12 coils, 192^3, 7.7 M of 30.7 M replicas, us): CB NU kLight 4 2 8:
 // 33.8 / 1137; 4 1 16: 46.7 / 1252; 4 4 16: 40.1 / 1134; 6 2 8: 33.9 / 1205;
 // 4 4 4: 42.5 / 1530; atomics per replica after a clearing pass: 85 / 3240.
-template <int NK, int CB, int NU, bool SUB>
+// NB bricks a block, their ranges loaded together: where most cells are empty a
+// block is little more than that latency (153^3, 2 cells of 100 with a replica,
+// 4 / 8 / 16 coils: NB 1 61 / 106 / 206 us, 2 55 / 93 / 165, 4 56 / 94 / 169;
+// clearing the grid and skipping the empty cells 60 / 101 / 181; 128^3, a
+// replica a cell, 8 coils: 183, 187, 202).
+template <int NK, int CB, int NU, bool SUB, int NB>
 __global__ void __launch_bounds__(kCellThreads)
     cell_sum_kernel(const float2* __restrict__ y, const uint32_t* __restrict__ start, const uint32_t* __restrict__ src,
                     const float* __restrict__ w, const int32_t* __restrict__ tix, const float2* __restrict__ basis,
@@ -130,20 +135,28 @@ __global__ void __launch_bounds__(kCellThreads)
     }
     return;
   }
-  const int brick = blockIdx.x - seg_blocks;
-  const int bxy = cg.nb[1] * cg.nb[2];
-  const int bz = brick / bxy, by = (brick - bz * bxy) / cg.nb[2], bx = brick % cg.nb[2];
+  const int bxy = cg.nb[1] * cg.nb[2], bricks = bxy * cg.nb[0];
+  const int b0 = (blockIdx.x - seg_blocks) * NB;
   const int lx = threadIdx.x % cg.b[2], ly = threadIdx.x / cg.b[2];
-  const int z = bz * cg.b[0] + ly / cg.b[1], yy = by * cg.b[1] + ly % cg.b[1], x = bx * cg.b[2] + lx;
-  if (z >= cg.g[0] || yy >= cg.g[1] || x >= cg.g[2]) return;
-  const uint32_t* st = start + static_cast<int64_t>(brick) * kCellThreads + threadIdx.x;
-  const uint32_t s = st[0], e = st[1];
-  if (e - s > kLight) return;
-  for (int b = blockIdx.z; b < B; b += gridDim.z) {
-    const float2* yb = y + (static_cast<int64_t>(b) * C + c0) * R;
-    float2 acc[NK][CB] = {};
-    for (uint32_t i = s; i < e; i += NU) add(acc, yb, i, e, 1);
-    store(acc, b, u, G, (static_cast<int64_t>(z) * cg.g[1] + yy) * cg.g[2] + x);
+  uint32_t s[NB], e[NB];
+#pragma unroll
+  for (int q = 0; q < NB; ++q) {
+    const uint32_t* st = start + static_cast<int64_t>(b0 + q) * kCellThreads + threadIdx.x;
+    s[q] = b0 + q < bricks ? st[0] : 0;
+    e[q] = b0 + q < bricks ? st[1] : 0xffffffffu;  // no brick: as a long list, left out
+  }
+#pragma unroll
+  for (int q = 0; q < NB; ++q) {
+    const int brick = b0 + q;
+    const int bz = brick / bxy, by = (brick - bz * bxy) / cg.nb[2], bx = brick % cg.nb[2];
+    const int z = bz * cg.b[0] + ly / cg.b[1], yy = by * cg.b[1] + ly % cg.b[1], x = bx * cg.b[2] + lx;
+    if (z >= cg.g[0] || yy >= cg.g[1] || x >= cg.g[2] || e[q] - s[q] > kLight) continue;
+    for (int b = blockIdx.z; b < B; b += gridDim.z) {
+      const float2* yb = y + (static_cast<int64_t>(b) * C + c0) * R;
+      float2 acc[NK][CB] = {};
+      for (uint32_t i = s[q]; i < e[q]; i += NU) add(acc, yb, i, e[q], 1);
+      store(acc, b, u, G, (static_cast<int64_t>(z) * cg.g[1] + yy) * cg.g[2] + x);
+    }
   }
 }
 
@@ -288,7 +301,7 @@ int pgb_cell_sum(const void* y, const uint32_t* start, const uint32_t* src, cons
     constexpr int NK = 4, CB = 2, NU = 1;
     const int64_t ny = (C + CB - 1) / CB * ((K + NK - 1) / NK);
     PGB_REQUIRE(ny <= 65535, PGB_ERR_RANGE, "cell_sum: too many coils");
-    cell_sum_kernel<NK, CB, NU, true><<<dim3(static_cast<unsigned>(nx), static_cast<unsigned>(ny), zb), kCellThreads, 0, s>>>(
+    cell_sum_kernel<NK, CB, NU, true, 1><<<dim3(static_cast<unsigned>(nx), static_cast<unsigned>(ny), zb), kCellThreads, 0, s>>>(
         static_cast<const float2*>(y), start, src, w, tix, static_cast<const float2*>(basis), static_cast<int>(T),
         static_cast<float2*>(u), g, static_cast<int>(B), static_cast<int>(C), static_cast<int>(K), R, G,
         static_cast<const int4*>(seg), static_cast<int>(n_seg), static_cast<float2*>(part));
@@ -296,7 +309,11 @@ int pgb_cell_sum(const void* y, const uint32_t* start, const uint32_t* src, cons
     constexpr int CB = 4, NU = 2;
     const int64_t ny = (C + CB - 1) / CB;
     PGB_REQUIRE(ny <= 65535, PGB_ERR_RANGE, "cell_sum: too many coils");
-    cell_sum_kernel<1, CB, NU, false><<<dim3(static_cast<unsigned>(nx), static_cast<unsigned>(ny), zb), kCellThreads, 0, s>>>(
+    // fewer replicas than cells in 3-D: two bricks a block (the comment at the kernel)
+    const int nb = ndim == 3 && R < G ? 2 : 1;
+    auto k = nb == 2 ? cell_sum_kernel<1, CB, NU, false, 2> : cell_sum_kernel<1, CB, NU, false, 1>;
+    const int64_t blocks = nx - bricks + (bricks + nb - 1) / nb;
+    k<<<dim3(static_cast<unsigned>(blocks), static_cast<unsigned>(ny), zb), kCellThreads, 0, s>>>(
         static_cast<const float2*>(y), start, src, w, nullptr, nullptr, 0, static_cast<float2*>(u), g,
         static_cast<int>(B), static_cast<int>(C), 1, R, G, static_cast<const int4*>(seg), static_cast<int>(n_seg),
         static_cast<float2*>(part));
