@@ -909,6 +909,8 @@ def expand_order(idx: torch.Tensor, K: int, C: int, kw: int, always: bool = Fals
     (mean run, us in sample order / ordered): spiral, 16 coils 15.1, 185 / 47; radial, 8 coils, 10,201 operators
     5.0, 82 / 39; radial, 32 coils 6.3, 903 / 262; 14 coils 5.5, 41 / 25; 3-D radial, 12 and 8 coils 1.9,
     206 / 217 and 1.95, 459 / 452; 3,328 samples of 8 coils 1.9, 3.7 / 4.9.
+    9 coils, 27 of 32 lanes in sample order and 8-byte loads in this one, from runs of 4.5 (4.0: 0.95, 5.0: 1.25
+    times as fast).
     """
     R = int(idx.numel())
     ns = _lib.lib().pgb_grog_expand_chunk(R // kw, C, kw)
@@ -922,7 +924,7 @@ def expand_order(idx: torch.Tensor, K: int, C: int, kw: int, always: bool = Fals
               runs.data_ptr(), _lib.stream_ptr(idx.device))
     if always:
         return order, entry, runs
-    return (order, entry) if R >= 3 * int(runs) else None
+    return (order, entry) if R >= (4.5 if C == 9 else 3) * int(runs) else None
 
 
 # ---------------------------------------------------------------------------
@@ -1187,14 +1189,22 @@ class GrogInterpolator:
 
     def _expand_order(self, s: int, idx: torch.Tensor, C: int, kw: int):
         """Replicas of stack element ``s`` ordered by operator inside each chunk of samples, ``(order, entry)`` of
-        ``csrc/grog_expand.cu``, where that pays: ``None`` where a chunk's replicas hardly share operators."""
+        ``csrc/grog_expand.cu``, where that pays: ``None`` where a chunk's replicas hardly share operators.
+
+        Up to 6 coils an operator is a few sectors, and only a table that no L1 holds is worth the order (sample
+        order / ordered, 10,201 operators of 2 and 4 coils 1.28 to 1.84 and 1.16 to 2.1, 121 of them 0.71 to 0.84 and
+        0.86 to 0.94); of 5 and 6 coils only that of small plans (150 k replicas 1.46 and 1.56, 820 k 1.07 and 0.89,
+        3.8 M 0.89 and 0.94)."""
+        K, R = int(self._table_d.shape[0]), idx.numel()
+        if C <= 6 and (8 * K * C * C <= 128 * 2**10 or (C > 4 and R > 600_000)):
+            return None
         if C % 4 == 0 and self._table_d.data_ptr() % 32:
             return None  # a view: its rows are not whole 32-byte sectors
         key, orders = (s, C), self.__dict__.setdefault("_orders", {})
         if key not in orders:
             if torch.cuda.is_current_stream_capturing():
                 return None  # the decision reads back from the device
-            orders[key] = expand_order(idx, int(self._table_d.shape[0]), C, kw)
+            orders[key] = expand_order(idx, K, C, kw)
         return orders[key]
 
     # -- gridded output (fused kernel) ------------------------------------------
