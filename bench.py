@@ -552,11 +552,11 @@ def _cg_iter_bytes(grid, image, C: int) -> int:
     pass (those in and out, the PSF once), output pass (those and the maps in, image
     out), vector step (p, Ap, r, x in, r, x, p out).  Grids without line lengths: the
     expansion, two cuFFT transforms of two passes, PSF and combine on full planes."""
-    from pygrog_b200._toep import circulant_length
+    from pygrog_b200._toep import circulant_length, line_images
 
     img = int(np.prod(image))
     lens = [circulant_length(n, m) for n, m in zip(grid, image)]
-    if len(grid) == 2 and None not in lens:
+    if len(grid) == 2 and None not in lens and C <= line_images(grid, image):
         rows = C * image[0] * lens[1]
         return 8 * (4 * rows + 2 * C * img + 2 * img) + 4 * lens[0] * lens[1] + 7 * 8 * img
     G = int(np.prod(grid))

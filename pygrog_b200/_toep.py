@@ -18,6 +18,8 @@ from __future__ import annotations
 
 __all__ = ["GrogToeplitzOp"]
 
+import math
+
 import numpy as np
 import torch
 
@@ -35,10 +37,60 @@ def circulant_length(N: int, n: int) -> int | None:
     twice its width where it is not (cuFFT's Bluestein transform pads as far).
     Measured, application on cuFFT / on lines, us: 16 coils, 640 (image 320)
     147 / 57; 14 coils, 277 105 / 37; 8 coils, 300 34 / 32, 64 16 / 9, 900
-    151 / 119; a full image of 1024 loses (183 / 188) and keeps cuFFT.
+    151 / 119; a full image of 1024 loses (183 / 188) and keeps cuFFT.  Grids whose
+    own length cuFFT transforms well are exceptions: below.
     """
     fit = [L for L in line_lengths() if L >= 2 * n or (L == N and L < 1024)]
     return min(fit) if fit else None
+
+
+# Where an image is as wide as its grid, the circulant length is about twice the grid's and the planes of the lines
+# have four times its cells.  That still beats cuFFT on lengths with a prime factor above 31, but not on every
+# other one: which, depends on the kernels that cuFFT has for the length.  Measured on square grids of every length
+# from 150 to 512 without line FFTs and with factors up to 31 (time on cuFFT / on lines):
+#  - the scalar operator from 16 coil images on (20 to 32 coils): below 0.97 (500: 0.78, 361: 0.87, 196: 0.90); below
+#    16 coils 0.9 to 1.7, on the others 0.97 to 2.7;
+#  - with 2 to 5 components (6 and 16 coils), the matrix of every frequency on top: below 0.9 on average over the
+#    components (500: 0.61, 361: 0.67), 0.9 to 1.1, 1.1 to 1.2.  3 and 5 components, whose packed matrix is not
+#    whole float4s, are at 0.93 and 0.88 of that average, 2 and 4 at 1.06 and 1.15.
+_GRID_LENGTHS = frozenset((
+    196, 289, 324, 325, 343, 352, 361, 364, 368, 390, 392, 399, 414, 416, 425, 455, 462, 464, 484, 490, 495,
+    496, 500, 504, 510,
+))
+_GRID_LENGTHS_SUB = frozenset((
+    196, 200, 243, 248, 250, 252, 255, 260, 264, 270, 272, 273, 285, 289, 297, 300, 304, 306, 308, 315, 323,
+    324, 325, 330, 336, 338, 340, 342, 343, 345, 350, 351, 352, 357, 361, 363, 364, 368, 375, 378, 385, 390,
+    391, 392, 396, 399, 405, 408, 414, 416, 420, 425, 429, 437, 440, 441, 448, 450, 455, 459, 462, 464, 468,
+    483, 484, 486, 490, 495, 496, 500, 504, 507, 510,
+))
+_GRID_LENGTHS_SUB35 = frozenset((
+    150, 152, 156, 162, 165, 168, 169, 175, 176, 184, 190, 195, 198, 204, 208, 209, 210, 220, 221, 224, 225,
+    230, 231, 232, 234, 242, 245, 247, 253, 275, 276, 280, 299, 322, 341, 348, 372, 380, 435, 460, 475, 476, 494,
+))
+_GRID_LENGTHS_SUB5 = frozenset((
+    132, 136, 153, 170, 182, 189, 228, 261, 294, 312, 319, 403, 406, 456, 493,
+))
+
+
+def _twice(grid, image, lengths) -> bool:
+    """Both axes of a 2-D grid are among ``lengths`` and their circulant lengths about twice that."""
+    return len(grid) == 2 and all(
+        N in lengths and (circulant_length(N, n) or 0) >= 1.9 * N for N, n in zip(grid, image))
+
+
+def line_images(grid, image) -> float:
+    """Coil images up to which the scalar operator is faster on lines than on cuFFT transforms of the grid."""
+    return 15 if _twice(grid, image, _GRID_LENGTHS) else math.inf
+
+
+def line_components(grid, image, K: int) -> bool:
+    """Whether the operator of ``K`` components is faster on lines than on cuFFT transforms of the grid."""
+    lengths = _GRID_LENGTHS_SUB
+    if K in (3, 5):
+        lengths = lengths | _GRID_LENGTHS_SUB35
+    if K == 5:
+        lengths = lengths | _GRID_LENGTHS_SUB5
+    return not _twice(grid, image, lengths)
 
 
 def line_plan(psf: torch.Tensor, grid, image):
@@ -96,7 +148,11 @@ class GrogToeplitzOp:
             psf = psf.reshape(S, *self.grid_shape)
         # reference attribute: PSF on the centred grid
         self.psf = psf.reshape(*self.stack_shape, *self.grid_shape) if self.stack_shape else psf[0]
-        self._lines = line_plan(psf, self.grid_shape, self.image_shape)
+        self._line_images = line_images(self.grid_shape, self.image_shape)
+        smaps = sparse_fft.smaps
+        self._lines = None
+        if smaps is None or int(smaps.shape[0]) <= self._line_images:
+            self._lines = line_plan(psf, self.grid_shape, self.image_shape)
         self._psf3 = None  # 3-D: PSF (S, G) of pgb_toep3d
         if len(self.grid_shape) == 3 and self._stage._lines(self.device) is not None:
             self._psf3 = torch.empty(S, G, dtype=torch.float32, device=self.device)
@@ -104,7 +160,7 @@ class GrogToeplitzOp:
                 p = self._stage.to_fft_order(psf[s]).to(torch.float64).contiguous()
                 _lib.call("pgb_toep_slots", p.data_ptr(), self.grid_shape[0], G // self.grid_shape[0], 1.0 / G,
                           self._psf3[s].data_ptr(), _lib.stream_ptr(p.device))
-        elif self._lines is None:
+        elif self._lines is None or self._line_images < math.inf:
             self._psf_fft = (self._stage.to_fft_order(psf) * (1.0 / G)).reshape(S, G).contiguous()
 
     def _n_coils(self, x):
@@ -128,7 +184,7 @@ class GrogToeplitzOp:
                       st._g.ctypes.data, tw[1].ctypes.data, x.data_ptr() if damp else None, float(damp),
                       _lib.stream_ptr(x.device))
             return out
-        if self._lines is not None:
+        if self._lines is not None and B * C <= self._line_images:
             b, c = (B, C) if smaps is not None else (B * C, 1)
             line_normal(self._lines, s, x, smaps, out, b, c, 0, st.image_shape, damp)
             return out

@@ -38,7 +38,7 @@ import torch
 from .. import _ext, _lib
 from .._fftops import as_c64, made_now, with_torch
 from .._solve import SolveMixin
-from .._toep import line_normal, line_plan
+from .._toep import line_components, line_normal, line_plan
 
 
 class SubspaceProjection:
@@ -403,7 +403,9 @@ class SubspaceToeplitzOp:
                 psfs.append(pf.transpose(-2, -1).contiguous())  # P[g, k, k']
             P = torch.stack(psfs).reshape(S, *self.grid_shape, self.K, self.K)
         self.psf = P[0] if not self.stack_shape else P.reshape(*self.stack_shape, *self.grid_shape, self.K, self.K)
-        self._lines = line_plan(_pack_hermitian(P), self.grid_shape, self.image_shape) if 1 < self.K <= _LINE_K else None
+        self._lines = None
+        if 1 < self.K <= _LINE_K and line_components(self.grid_shape, self.image_shape, self.K):
+            self._lines = line_plan(_pack_hermitian(P), self.grid_shape, self.image_shape)
         if self._lines is not None:
             return
         # FFT order, 1/G of the two unscaled transforms folded in
