@@ -9,8 +9,8 @@ iteration -- ``Ap = A^H A p + damp p`` (Toeplitz or fused forward/adjoint),
 FP64 ``<p, Ap>``, x/r update, FP64 ``|r|^2`` with the relative-residual test,
 p update -- with every scalar kept in device memory and a device flag
 replacing the host-side ``break``.  Without a callback a few iterations (and
-one, for the rest) are captured in a CUDA graph and replayed ``max_iter``
-iterations long: no host synchronisation inside the loop.  Other duck-typed operators use the
+one, for the rest, from the second solve on) are captured in a CUDA graph and
+replayed ``max_iter`` iterations long: no host synchronisation inside the loop.  Other duck-typed operators use the
 reference recurrence with torch tensors (inner products in FP64).
 """
 
@@ -87,6 +87,7 @@ class DeviceCG:
         _lib.call("pgb_dot_f64", self.r.data_ptr(), None, self.n, self.scratch.data_ptr(),
                   self.scal.data_ptr(), 0, 2, st)
         self.graphs: dict = {}  # iterations -> graph
+        self.solves = 0
 
     def reset(self, AHb: torch.Tensor, x0=None):
         """Start a new solve in the same buffers (a captured iteration graph stays valid)."""
@@ -139,13 +140,17 @@ class DeviceCG:
 
     def run(self, max_iter: int, callback: Callable | None = None, use_graph: bool = True):
         if callback is None and use_graph and max_iter > 1:
-            left = int(max_iter)
+            left, first, self.solves = int(max_iter), self.solves == 0, self.solves + 1
             for iters in (_CG_ITERS_PER_GRAPH, 1):
                 if left >= iters and iters not in self.graphs:
+                    if first and iters == 1:
+                        break  # a capture costs more than the launches of these few; the next solve makes it
                     self.capture(iters)
                 while left >= iters:
                     self.graphs[iters].replay()
                     left -= iters
+            for _ in range(left):
+                self.step()
             return self.x
         for k in range(max_iter):
             self.step()
