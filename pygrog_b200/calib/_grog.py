@@ -655,22 +655,22 @@ class GrogGridder:
         They write and read the shifted replicas once more than the others but fill the GPU on any trajectory, so
         they win where the others are short of work, and lose at length to the brick kernels, which read no
         operator from L2 (a run of 4 halves that traffic).  Measured (1,347 plans and batches, coils 4 to 32; time
-        of grid and degrid, other / ordered): brick kernels, 3-D, 12 coils: 29 k 2.33, 80 k 1.52, 144 k 1.17, 250 k
-        0.86, 1.2 M 0.62; 2-D, 8 coils, 10,201 operators: 33 k 2.00, 2 frames 1.39, 4 frames 1.15, 16 frames 0.85,
-        179 k 0.95; spirals of 8 coils, runs of 12 and 8: 197 k 1.44, 246 k 1.21; 2-D, 16 coils, run 2.9: 90 k
-        1.40, 179 k 0.95.  Where no more than the smallest 3-D brick fits beside the tables (13 coils), in which most
-        of the work is on its faces, the brick kernels lose throughout: 144 k 1.59, 2.7 M 1.09, 16 frames of it 1.01.
+        of grid and degrid, other / ordered): brick kernels, 3-D, 12 coils: 29 k 2.33, 80 k 1.55, 144 k 1.19, 250 k
+        0.86, 1.2 M 0.63; 2-D, 8 coils, 10,201 operators: 33 k 2.09, 2 frames 1.41, 4 frames 1.19, 16 frames 0.87,
+        179 k 1.00; spirals of 8 coils, runs of 12 and 8: 197 k 1.51, 246 k 1.25; 2-D, 16 coils, run 2.9: 90 k
+        1.41, 179 k 0.97.  Where no more than the smallest 3-D brick fits beside the tables (13 coils), in which most
+        of the work is on its faces, the brick kernels lose throughout: 144 k 1.61, 2.7 M 1.12, 16 frames of it 1.05.
         The table through L1/L2 loses to short runs of whole sectors (C a multiple of 8) and to long runs
-        throughout (16 / 24 / 32 coils in 3-D at 1.2 M 1.50 / 1.62 / 1.57; 2-D above 1.15).  Else it wins at
-        length, the sooner the more lanes its groups of C fill: 15 coils 420 k 1.47, 800 k 0.82; 31 coils 420 k
-        1.06, 1.2 M 0.71; 20 coils 420 k 1.50, 2 frames 1.19, 1.2 M 0.97.
+        throughout (16 / 24 / 32 coils in 3-D at 1.2 M 1.42 / 1.50 / 1.46; 2-D above 1.15).  Else it wins at
+        length: 15 coils 420 k 1.49, 800 k 0.65; 20 coils 420 k 1.41, 2 frames 1.07, 1.2 M 0.89; 31 coils, 8-byte
+        loads of nearly 8 KB operators, 144 k 2.79, 2 frames 1.90, 420 k 0.81.
         """
         family, brick = other
         if family != "global":
             return math.inf if brick == self.BRICKS3[-1] else 256e3 if run >= 4 else 150e3
         if self.C % 8 == 0 or run >= 2.5:
             return math.inf
-        return 500e3 if 32 // self.C * self.C >= 28 else 1e6
+        return 300e3 if self.C >= 30 else 750e3
 
     def _init_ordered(self, target_idx, interp_idx, rep_weight, kw, grid_shape, table, factors, other) -> bool:
         """The plan's valid replicas, ascending by sample: their operators' order (``csrc/grog_expand.cu``), the
@@ -909,8 +909,6 @@ def expand_order(idx: torch.Tensor, K: int, C: int, kw: int, always: bool = Fals
     (mean run, us in sample order / ordered): spiral, 16 coils 15.1, 185 / 47; radial, 8 coils, 10,201 operators
     5.0, 82 / 39; radial, 32 coils 6.3, 903 / 262; 14 coils 5.5, 41 / 25; 3-D radial, 12 and 8 coils 1.9,
     206 / 217 and 1.95, 459 / 452; 3,328 samples of 8 coils 1.9, 3.7 / 4.9.
-    9 coils, 27 of 32 lanes in sample order and 8-byte loads in this one, from runs of 4.5 (4.0: 0.95, 5.0: 1.25
-    times as fast).
     """
     R = int(idx.numel())
     ns = _lib.lib().pgb_grog_expand_chunk(R // kw, C, kw)
@@ -924,7 +922,7 @@ def expand_order(idx: torch.Tensor, K: int, C: int, kw: int, always: bool = Fals
               runs.data_ptr(), _lib.stream_ptr(idx.device))
     if always:
         return order, entry, runs
-    return (order, entry) if R >= (4.5 if C == 9 else 3) * int(runs) else None
+    return (order, entry) if R >= 3 * int(runs) else None
 
 
 # ---------------------------------------------------------------------------
@@ -1192,9 +1190,9 @@ class GrogInterpolator:
         ``csrc/grog_expand.cu``, where that pays: ``None`` where a chunk's replicas hardly share operators.
 
         Up to 6 coils an operator is a few sectors, and only a table that no L1 holds is worth the order (sample
-        order / ordered, 10,201 operators of 2 and 4 coils 1.28 to 1.84 and 1.16 to 2.1, 121 of them 0.71 to 0.84 and
-        0.86 to 0.94); of 5 and 6 coils only that of small plans (150 k replicas 1.46 and 1.56, 820 k 1.07 and 0.89,
-        3.8 M 0.89 and 0.94)."""
+        order / ordered, 10,201 operators of 2 / 3 / 4 coils 1.2 to 1.7 / 1.04 to 1.7 / 1.2 to 1.8, 121 of them 0.98 to 1 /
+        0.91 to 1 / 1; of 1 coil 0.8 to 1); of 5 and 6 coils only that of small plans (150 k replicas 1.47 and 1.64,
+        575 k 1.27 and 1.18, 820 k and 3.8 M 0.98 and 0.99; 121 operators 0.93 to 1.01)."""
         K, R = int(self._table_d.shape[0]), idx.numel()
         if C <= 6 and (8 * K * C * C <= 128 * 2**10 or (C > 4 and R > 600_000)):
             return None

@@ -77,7 +77,7 @@ __device__ __forceinline__ float2 row_dot(const float2* __restrict__ T, const fl
 // away what they keep (errors up to 3.6 times theirs).  Twice the products, but
 // on few operators: 33 k replicas of 8 coils (10,201 operators of 2 x 101
 // factors) 26 / 22 us for grid / degrid against 24 / 19 with the whole table,
-// 1.2 M of 11 coils in 3-D 416 / 449 against 572 / 643, of 12 coils 498 / 550
+// 1.2 M of 11 coils in 3-D 400 / 445 against 572 / 643, of 12 coils 481 / 540
 // against 444 / 541.
 struct ShiftTable {
   const float2* table;
@@ -132,7 +132,10 @@ __global__ void __launch_bounds__(kExpThreads, 2)
       if constexpr (FACT) at = tb.swap ? at / tb.n : at % tb.n;
       const float2* T = (FACT && !tb.swap ? tb.second : tb.table) + (static_cast<int64_t>(at) * C + g0) * C;
 #pragma unroll 4  // the operator rows of four coils in flight
-      for (int co = 0; co < ng; ++co, T += C) stage[co * SR + l] = ok ? row_dot<C, PART>(T, x) : make_float2(0.f, 0.f);
+      for (int co = 0; co < ng; ++co, T += C) {
+        const float2 y = row_dot<C, PART>(T, x);  // in every lane: a branch here would keep the rows' loads apart
+        stage[co * SR + l] = ok ? y : make_float2(0.f, 0.f);
+      }
     }
     __syncthreads();
     for (int co = 0; co < ng; ++co)

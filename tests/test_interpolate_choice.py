@@ -15,8 +15,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("C,precision,ordered", [(1, 1, False), (2, 1, False), (4, 1, False), (6, 1, False), (8, 1, True),
                                                  (2, 2, True), (4, 2, True), (5, 2, True), (6, 2, True)])
 def test_few_coils(cuda, C, precision, ordered):
-    """Measured, sample order / ordered: 121 operators of 1 / 2 / 4 / 6 coils 0.67 / 0.71 / 0.86 / 0.95, of 8 1.35;
-    10,201 of 2 / 4 / 5 / 6 on a small plan 1.84 / 2.09 / 1.46 / 1.56."""
+    """Measured, sample order / ordered: 121 operators of 1 / 2 / 4 / 6 coils 0.8 / 0.98 / 1 / 0.95, of 8 1.35;
+    10,201 of 2 / 4 / 5 / 6 on a small plan 1.73 / 1.84 / 1.47 / 1.64."""
     rng = np.random.default_rng(C)
     cplx = lambda *s: (rng.standard_normal(s) + 1j * rng.standard_normal(s)).astype(np.complex64)  # noqa: E731
     n, spokes, readout = 64, 12, 300
