@@ -163,6 +163,10 @@ class GrogToeplitzOp:
         elif self._lines is None or self._line_images < math.inf:
             self._psf_fft = (self._stage.to_fft_order(psf) * (1.0 / G)).reshape(S, G).contiguous()
 
+    def __setstate__(self, state):
+        # saved before: cuFFT alone, or lines wherever they were made
+        self.__dict__.update({"_line_images": math.inf, "_lines": None, "_psf3": None, **state})
+
     def _n_coils(self, x):
         sm = self.sparse_fft.smaps
         return int(sm.shape[0]) if sm is not None else int(x.shape[1])

@@ -645,6 +645,13 @@ class GrogGridder:
         self.plan = BrickPlan(target_idx, interp_idx, rep_weight, kw, grid_shape, **kwargs)
         self.adj_plan = self.plan
 
+    def __setstate__(self, state):
+        """Ordered gridders saved before they knew factors and other families: the whole table, for every batch."""
+        if state.get("mode") == "ordered" and "ops" not in state:
+            state = {**state, "ops": [state["table"], None], "ops_h": [state["table_h"], None], "n_outer": 1,
+                     "K": int(state["table"].shape[0]), "max_batch": math.inf, "_other": None, "_make_other": None}
+        self.__dict__.update(state)
+
     def _can_order(self, target_idx, kw, grid_shape, K) -> bool:
         return (self.C <= 32 and int(np.prod(grid_shape)) < 2**31 and target_idx.numel() < 2**31 and K < 2**31 - 1)
 

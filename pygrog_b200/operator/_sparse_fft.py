@@ -44,7 +44,7 @@ class _StackArrays:
         self.w = sw_nat.to(torch.float32).contiguous()
         self.w_fwd = (self.w * stage.ortho).contiguous()
         self.R = int(idx_nat.numel())
-        self._stage, self._lists = stage, None
+        self._stage, self._lists = stage, None  # lists by cell and their weights
 
     def by_cell(self) -> tuple:
         """The replicas by cell, for the adjoint, and their weights."""
@@ -134,6 +134,9 @@ class SparseFFT(SolveMixin):
         self.toeplitz = bool(toeplitz)
         self._toep_op = None
         self._arrays = None
+
+    def __setstate__(self, state):
+        self.__dict__.update(state, _arrays=None)  # made at the first call
 
     # ------------------------------------------------------------------
     def _stack_arrays_dev(self, s: int) -> _StackArrays:

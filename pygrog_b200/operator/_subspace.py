@@ -125,6 +125,9 @@ class SubspaceSparseFFT(SolveMixin):
         self._w2 = {}
         self._lists = {}
 
+    def __setstate__(self, state):
+        self.__dict__.update(state, _lists={})  # made at the first call
+
     # -- helpers -----------------------------------------------------------------
     def _require_smaps(self):
         if self._base.smaps is None:
@@ -411,6 +414,9 @@ class SubspaceToeplitzOp:
         # FFT order, 1/G of the two unscaled transforms folded in
         Pf = torch.fft.ifftshift(P, dim=tuple(range(1, 1 + len(self.grid_shape))))
         self._psf_fft = (Pf.reshape(S, st.G, self.K, self.K) * (1.0 / st.G)).contiguous()
+
+    def __setstate__(self, state):
+        self.__dict__.update({"_lines": None, **state})  # saved before the lines: cuFFT
 
     def _apply_frames(self, x: torch.Tensor, s: int, out: torch.Tensor, damp: float = 0.0) -> torch.Tensor:
         """x (Bt, K, *image) on the device -> out (same shape)."""
