@@ -242,10 +242,14 @@ def check_tc_timeouts(what: str) -> None:
         )
 
 
+_NUMBERED = {torch.device("cuda", i): i for i in range(64)}  # asking a device for its type costs more than the look
+
+
 def stream_ptr(device=None) -> int:
     """The current stream of ``device`` (anything torch takes as one)."""
-    if isinstance(device, torch.device) and device.index is not None and device.type == "cuda":
-        return torch._C._cuda_getCurrentRawStream(device.index)
+    index = _NUMBERED.get(device)
+    if index is not None:
+        return torch._C._cuda_getCurrentRawStream(index)
     return torch.cuda.current_stream(device).cuda_stream
 
 

@@ -1200,17 +1200,20 @@ class GrogInterpolator:
         order / ordered, 10,201 operators of 2 / 3 / 4 coils 1.2 to 1.7 / 1.04 to 1.7 / 1.2 to 1.8, 121 of them 0.98 to 1 /
         0.91 to 1 / 1; of 1 coil 0.8 to 1); of 5 and 6 coils only that of small plans (150 k replicas 1.47 and 1.64,
         575 k 1.27 and 1.18, 820 k and 3.8 M 0.98 and 0.99; 121 operators 0.93 to 1.01)."""
-        K, R = int(self._table_d.shape[0]), idx.numel()
-        if C <= 6 and (8 * K * C * C <= 128 * 2**10 or (C > 4 and R > 600_000)):
-            return None
-        if C % 4 == 0 and self._table_d.data_ptr() % 32:
-            return None  # a view: its rows are not whole 32-byte sectors
         key, orders = (s, C), self.__dict__.setdefault("_orders", {})
-        if key not in orders:
-            if torch.cuda.is_current_stream_capturing():
+        order = orders.get(key, False)
+        if order is False:
+            K, R = int(self._table_d.shape[0]), idx.numel()
+            if C <= 6 and (8 * K * C * C <= 128 * 2**10 or (C > 4 and R > 600_000)):
+                order = None
+            elif torch.cuda.is_current_stream_capturing():
                 return None  # the decision reads back from the device
-            orders[key] = expand_order(idx, K, C, kw)
-        return orders[key]
+            else:
+                order = expand_order(idx, K, C, kw)
+            orders[key] = order
+        if order is not None and C % 4 == 0 and self._table_d.data_ptr() % 32:
+            return None  # a view: its rows are not whole 32-byte sectors
+        return order
 
     # -- gridded output (fused kernel) ------------------------------------------
     def _density_grid(self) -> torch.Tensor:

@@ -174,14 +174,14 @@ class MaskedFFT(SolveMixin):
     @with_torch
     def normal(self, image):
         if self.toeplitz:
-            return self._toeplitz()(image)
+            return (self._toep_op or self._toeplitz())(image)
         return self.adjoint(self.forward(image))
 
     def _normal_into(self, x, out, damp: float = 0.0):
         if self.stack_shape:
             raise NotImplementedError("device CG loop covers unstacked operators")
         if self.toeplitz:
-            return self._toeplitz()._apply_into(x, out, damp)
+            return (self._toep_op or self._toeplitz())._apply_into(x, out, damp)
         y = self.adjoint(self.forward(x))
         out.copy_(y + damp * x if damp else y)
         return out

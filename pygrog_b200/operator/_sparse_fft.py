@@ -277,7 +277,7 @@ class SparseFFT(SolveMixin):
     def normal(self, image):
         """``A^H A image`` (Toeplitz PSF when ``self.toeplitz``, else adjoint(forward))."""
         if self.toeplitz:
-            return self._toeplitz()(image)
+            return (self._toep_op or self._toeplitz())(image)
         return self.adjoint(self.forward(image))
 
     def _normal_into(self, x: torch.Tensor, out: torch.Tensor, damp: float = 0.0) -> torch.Tensor:
@@ -286,7 +286,7 @@ class SparseFFT(SolveMixin):
         if self.stack_shape:
             raise NotImplementedError("device CG loop covers unstacked operators")
         if self.toeplitz:
-            return self._toeplitz()._apply_into(x, out, damp)
+            return (self._toep_op or self._toeplitz())._apply_into(x, out, damp)
         C = self._n_coils(x.shape[0] if x.ndim > len(self.image_shape) else 1)
         k = self._forward_core(x.reshape(1, *x.shape), 0, C)
         st = self._stage
@@ -299,7 +299,7 @@ class SparseFFT(SolveMixin):
         if self.stack_shape:
             raise NotImplementedError("frame-batched normal operator covers unstacked operators")
         if self.toeplitz:
-            return self._toeplitz()._apply_frames(x, 0, out, damp)
+            return (self._toep_op or self._toeplitz())._apply_frames(x, 0, out, damp)
         F = int(x.shape[0])
         C = self._n_coils(x.shape[1] if x.ndim > len(self.image_shape) + 1 else 1)
         k = self._forward_core(x, 0, C)

@@ -243,7 +243,7 @@ class SubspaceSparseFFT(SolveMixin):
     def normal(self, coeffs):
         """``A^H A coeffs`` (Toeplitz K x K PSF when ``self.toeplitz``)."""
         if self.toeplitz:
-            return self._toeplitz()(coeffs)
+            return (self._toep_op or self._toeplitz())(coeffs)
         return self.adjoint(self.forward(coeffs))
 
     def _normal_frames_into(self, x: torch.Tensor, out: torch.Tensor, damp: float = 0.0) -> torch.Tensor:
@@ -251,7 +251,7 @@ class SubspaceSparseFFT(SolveMixin):
         if self.stack_shape:
             raise NotImplementedError("frame-batched normal operator covers unstacked operators")
         if self.toeplitz:
-            return self._toeplitz()._apply_frames(x, 0, out, damp)
+            return (self._toep_op or self._toeplitz())._apply_frames(x, 0, out, damp)
         y = self._adjoint_core(self._forward_core(x, 0), 0)
         torch.add(y, x, alpha=damp, out=out) if damp else out.copy_(y)
         return out
@@ -261,7 +261,7 @@ class SubspaceSparseFFT(SolveMixin):
         if self.stack_shape:
             raise NotImplementedError("device CG loop covers unstacked operators")
         if self.toeplitz:
-            return self._toeplitz()._apply_frames(x.unsqueeze(0), 0, out.unsqueeze(0), damp)
+            return (self._toep_op or self._toeplitz())._apply_frames(x.unsqueeze(0), 0, out.unsqueeze(0), damp)
         y = self._adjoint_core(self._forward_core(x.unsqueeze(0), 0), 0)
         torch.add(y[0], x, alpha=damp, out=out) if damp else out.copy_(y[0])
         return out
