@@ -24,7 +24,7 @@ import numpy as np
 import torch
 
 from . import _ext, _lib
-from ._fftops import FFTStage, as_c64, compute_device, line_lengths
+from ._fftops import FFTStage, as_c64, compute_device, line_lengths, made_now
 
 
 def circulant_length(N: int, n: int) -> int | None:
@@ -160,12 +160,17 @@ class GrogToeplitzOp:
                 p = self._stage.to_fft_order(psf[s]).to(torch.float64).contiguous()
                 _lib.call("pgb_toep_slots", p.data_ptr(), self.grid_shape[0], G // self.grid_shape[0], 1.0 / G,
                           self._psf3[s].data_ptr(), _lib.stream_ptr(p.device))
-        elif self._lines is None or self._line_images < math.inf:
-            self._psf_fft = (self._stage.to_fft_order(psf) * (1.0 / G)).reshape(S, G).contiguous()
+        self._psf_fft = None  # PSF (S, G) of the cuFFT transforms
+        if self._psf3 is None and self._lines is None:
+            self._psf_fft = self._grid_psf()
+
+    def _grid_psf(self) -> torch.Tensor:
+        psf = self.psf.reshape(-1, *self.grid_shape)
+        return (self._stage.to_fft_order(psf) * (1.0 / self._stage.G)).reshape(-1, self._stage.G).contiguous()
 
     def __setstate__(self, state):
         # saved before: cuFFT alone, or lines wherever they were made
-        self.__dict__.update({"_line_images": math.inf, "_lines": None, "_psf3": None, **state})
+        self.__dict__.update({"_line_images": math.inf, "_lines": None, "_psf3": None, "_psf_fft": None, **state})
 
     def _n_coils(self, x):
         sm = self.sparse_fft.smaps
@@ -195,7 +200,12 @@ class GrogToeplitzOp:
         u = torch.empty(B, C, *st.grid_shape, dtype=torch.complex64, device=x.device)
         st.expand(x, smaps, u, B, C, 1.0, x_has_coils=smaps is None)
         U = st.fft(u)
-        st.psf_apply(U, self._psf_fft[s], B * C, st.G)
+        psf = self._psf_fft
+        if psf is None:  # more coil images than lines are worth, for the first time
+            psf = self._grid_psf()
+            if made_now(self.device):
+                self._psf_fft = psf
+        st.psf_apply(U, psf[s], B * C, st.G)
         V = st.ifft(U)
         st.combine(V, smaps, out, B, C, 1.0, add=x if damp else None, add_scale=damp)
         return out
