@@ -655,9 +655,10 @@ class GrogGridder:
     def _can_order(self, target_idx, kw, grid_shape, K) -> bool:
         return (self.C <= 32 and int(np.prod(grid_shape)) < 2**31 and target_idx.numel() < 2**31 and K < 2**31 - 1)
 
-    def _order_limit(self, other: tuple, run: float) -> float:
+    def _order_limit(self, other: tuple, run: float, density: float = math.inf, replicas: int = 0) -> float:
         """Replicas (frames times the plan's) up to which the ordered kernels are the faster ones, against the family
-        and brick ``other`` that the plan would have without them; ``run``: replicas that share an operator in a chunk.
+        and brick ``other`` that the plan would have without them; ``run``: replicas that share an operator in a chunk,
+        ``density``: the plan's ``replicas`` a cell of a 3-D grid.
 
         They write and read the shifted replicas once more than the others but fill the GPU on any trajectory, so
         they win where the others are short of work, and lose at length to the brick kernels, which read no
@@ -667,6 +668,9 @@ class GrogGridder:
         179 k 1.00; spirals of 8 coils, runs of 12 and 8: 197 k 1.51, 246 k 1.25; 2-D, 16 coils, run 2.9: 90 k
         1.41, 179 k 0.97.  Where no more than the smallest 3-D brick fits beside the tables (13 coils), in which most
         of the work is on its faces, the brick kernels lose throughout: 144 k 1.61, 2.7 M 1.12, 16 frames of it 1.05.
+        Sparse 3-D plans leave the bricks with little but their tiles: to 0.13 replicas a cell the brick kernels lose
+        at any size (8 / 12 coils: 137 k 1.50 / 1.75, 432 k 1.23 / 1.36, in batches the same), to 0.18 up to 400 k (344 k
+        1.10 / 1.17); of 4 and 6 coils to 0.18 single frames (1.10 to 1.8; batches 0.74 to 1.6).
         The table through L1/L2 loses to short runs of whole sectors (C a multiple of 8) and to long runs
         throughout (16 / 24 / 32 coils in 3-D at 1.2 M 1.42 / 1.50 / 1.46; 2-D above 1.15).  Else it wins at
         length: 15 coils 420 k 1.49, 800 k 0.65; 20 coils 420 k 1.41, 2 frames 1.07, 1.2 M 0.89; 31 coils, 8-byte
@@ -674,7 +678,10 @@ class GrogGridder:
         """
         family, brick = other
         if family != "global":
-            return math.inf if brick == self.BRICKS3[-1] else 256e3 if run >= 4 else 150e3
+            if brick == self.BRICKS3[-1] or (density <= 0.13 and self.C >= 8):
+                return math.inf
+            dense = 256e3 if run >= 4 else 150e3
+            return dense if density > 0.18 else 400e3 if self.C >= 8 else max(dense, replicas)
         if self.C % 8 == 0 or run >= 2.5:
             return math.inf
         return 300e3 if self.C >= 30 else 750e3
@@ -690,12 +697,13 @@ class GrogGridder:
             raise ValueError("ordered kernels need C <= 32 and grids, replica counts and tables below 2^31")
         r = torch.nonzero(tgt >= 0).squeeze(1)
         V, C, K = int(r.numel()), self.C, int(table.shape[0])
-        limit = math.inf if other is None else self._order_limit(other, math.inf)
+        density = V / math.prod(grid_shape) if len(grid_shape) == 3 else math.inf
+        limit = math.inf if other is None else self._order_limit(other, math.inf, density, V)
         if V > limit:
             return False
         order, entry, runs = expand_order(interp_idx.reshape(-1)[r], K, C, 1, always=True)
         if other is not None:
-            limit = self._order_limit(other, V / max(1, int(runs)))
+            limit = self._order_limit(other, V / max(1, int(runs)), density, V)
         if V > limit:
             return False
         self.max_batch = math.inf if V == 0 else limit / V

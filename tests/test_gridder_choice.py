@@ -35,6 +35,20 @@ def test_rule_follows_the_measurements(work, C, other, run, gain):
     assert _limit(C, other, math.inf) >= _limit(C, other, run)  # the bound before the runs are known
 
 
+# replicas of the plan, frames, coils, replicas a cell
+@pytest.mark.parametrize("V,frames,C,density,gain", [
+    (137e3, 16, 8, 0.07, 1.53), (432e3, 4, 12, 0.11, 1.27), (388e3, 1, 8, 0.13, 1.17), (344e3, 1, 12, 0.16, 1.17),
+    (516e3, 1, 8, 0.25, 0.86), (344e3, 2, 4, 0.16, 0.91), (388e3, 1, 4, 0.13, 1.25), (388e3, 4, 4, 0.13, 0.96), (188e3, 1, 6, 0.13, 1.17), (188e3, 2, 6, 0.13, 0.92),
+    (1080e3, 1, 12, 0.26, 0.83),
+])
+def test_rule_for_sparse_3d_plans(V, frames, C, density, gain):
+    g = GrogGridder.__new__(GrogGridder)
+    g.C = C
+    limit = g._order_limit(("v8", (8, 8, 8)), 1.1, density, V)
+    assert (V * frames <= limit) == (gain > 1)
+    assert g._order_limit(("v8", (8, 8, 8)), math.inf, density, V) >= limit
+
+
 def _gridder(dev, ndim, n, spokes, readout, C, **kw):
     rng = np.random.default_rng(n)
     cplx = lambda *s: (rng.standard_normal(s) + 1j * rng.standard_normal(s)).astype(np.complex64)  # noqa: E731
