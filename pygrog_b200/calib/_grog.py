@@ -665,7 +665,7 @@ class GrogGridder:
         operator from L2 (a run of 4 halves that traffic).  Measured (1,347 plans and batches, coils 4 to 32; time
         of grid and degrid, other / ordered): brick kernels, 3-D, 12 coils: 29 k 2.33, 80 k 1.55, 144 k 1.19, 250 k
         0.86, 1.2 M 0.63; 2-D, 8 coils, 10,201 operators: 33 k 2.09, 2 frames 1.41, 4 frames 1.19, 16 frames 0.87,
-        179 k 1.00; spirals of 8 coils, runs of 12 and 8: 197 k 1.51, 246 k 1.25; 2-D, 16 coils, run 2.9: 90 k
+        179 k 1.00; spirals of 9 coils, run 12: 197 k 1.37, 2 frames 1.36, run 4.4: 246 k 1.20, 2 frames 1.04; 2-D, 16 coils, run 2.9: 90 k
         1.41, 179 k 0.97.  Where no more than the smallest 3-D brick fits beside the tables (13 coils), in which most
         of the work is on its faces, the brick kernels lose throughout: 144 k 1.61, 2.7 M 1.12, 16 frames of it 1.05.
         Sparse 3-D plans leave the bricks with little but their tiles: to 0.13 replicas a cell the brick kernels lose
@@ -680,7 +680,7 @@ class GrogGridder:
         if family != "global":
             if brick == self.BRICKS3[-1] or (density <= 0.13 and self.C >= 8):
                 return math.inf
-            dense = 256e3 if run >= 4 else 150e3
+            dense = 400e3 if run >= 6 else 256e3 if run >= 4 else 150e3
             return dense if density > 0.18 else 400e3 if self.C >= 8 else max(dense, replicas)
         if self.C % 8 == 0 or run >= 2.5:
             return math.inf

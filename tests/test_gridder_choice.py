@@ -24,7 +24,8 @@ def _limit(C, other, run):
     (600e3, 13, ("v8", (2, 4, 8)), 1.2, 1.5), (43e6, 13, ("v8", (2, 4, 8)), 1.29, 1.05),
     (33e3, 8, ("v8", (1, 16, 32)), 1.01, 2.09), (524e3, 8, ("v8", (1, 16, 32)), 1.01, 0.87),
     (179e3, 11, ("v8", (1, 16, 32)), 1.04, 0.80), (197e3, 8, ("v8", (1, 16, 32)), 12.1, 1.51),
-    (246e3, 8, ("v8", (1, 16, 32)), 8.4, 1.25), (538e3, 16, ("v8", (1, 16, 32)), 5.6, 0.93),
+    (246e3, 8, ("v8", (1, 16, 32)), 8.4, 1.25), (394e3, 9, ("v8", (1, 16, 32)), 12.1, 1.36),
+    (358e3, 13, ("v8", (1, 16, 32)), 5.2, 0.87), (538e3, 16, ("v8", (1, 16, 32)), 5.6, 0.93),
     (1.2e6, 16, ("global", None), 1.27, 1.42), (3e6, 32, ("global", None), 1.15, 1.35),
     (288e3, 31, ("global", None), 1.11, 1.90), (420e3, 31, ("global", None), 1.16, 0.81),
     (800e3, 15, ("global", None), 1.25, 0.65), (420e3, 20, ("global", None), 1.21, 1.41),
